@@ -632,6 +632,17 @@ struct pbf_adjoint {
     // Scratch of one step: keys, sort buffers, composed permutations, the
     // cell table, component arrays and the predicted / projected positions.
     DeviceBuffer keys, skeys, akeys, aidx, orgs, first, soa, xs0, vin, pn, scratch, status;
+    // Counting sort of the rebuilds (empty: the radix sort); akeys holds the
+    // arrival places, aidx the cells' lists.
+    DeviceBuffer bin_count;
+    CellBins cell_bins() const {
+        CellBins b;
+        if (bin_count.get()) {
+            b.count = bin_count.as<uint32_t>();
+            b.place = akeys.as<uint32_t>();
+        }
+        return b;
+    }
     // Tape of one segment (`every` step slots), see the accessors below.
     DeviceBuffer tf4, tu32, tlam, tnb, tcn, tmv;
     // States in particle-id order: slot j holds (x, v) entering step j of a
@@ -779,6 +790,10 @@ struct pbf_adjoint {
         aidx.allocate(u4b);
         orgs.allocate(2 * u4b);
         first.allocate((cells + 1) * sizeof(int));
+        if (bins_apply(n, cells))
+            bin_count.allocate(bin_count_words(cells) * sizeof(uint32_t));
+        else
+            bin_count = DeviceBuffer();
         soa.allocate(3 * soa_stride() * sizeof(float));
         scratch.allocate(sort_scratch_bytes(static_cast<int>(n)));
         status.allocate(sizeof(unsigned));
@@ -803,7 +818,7 @@ struct pbf_adjoint {
         acc_c.allocate(n * sizeof(double));
         // Index data starts zeroed, so no index read after a failed step is
         // ever out of range.
-        for (DeviceBuffer* b : {&tnb, &tcn, &tu32, &tmv, &orgs, &first, &keys})
+        for (DeviceBuffer* b : {&tnb, &tcn, &tu32, &tmv, &orgs, &first, &keys, &aidx})
             cuda_check(cudaMemsetAsync(b->get(), 0, b->bytes(), stream));
         cuda_check(cudaStreamSynchronize(stream));
         ckpt = DeviceBuffer();
@@ -870,6 +885,14 @@ struct pbf_adjoint {
         const int N = static_cast<int>(n);
         unsigned* sp = status.as<unsigned>();
         float* s0 = soa.as<float>();
+        if (bin_count.get()) {
+            launch_bin_order(cell_bins(), keys.as<uint32_t>(), first.as<int>(), aidx.as<uint32_t>(),
+                             N, cells, sp, stream);
+            launch_bin_gather(cell_bins(), aidx.as<uint32_t>(), keys.as<uint32_t>(),
+                              first.as<int>(), cells, src, dst, org_in, org_out, rel, s0,
+                              s0 + soa_stride(), s0 + 2 * soa_stride(), N, sp, stream);
+            return;
+        }
         launch_sort(plan, keys.as<uint32_t>(), skeys.as<uint32_t>(), rel, akeys.as<uint32_t>(),
                     aidx.as<uint32_t>(), scratch.get(), sp, stream);
         launch_gather_first(rel, src, dst, org_in, org_out, s0, s0 + soa_stride(),
@@ -886,8 +909,8 @@ struct pbf_adjoint {
         float* s0 = soa.as<float>();
         uint32_t* oa = orgs.as<uint32_t>();
         uint32_t* ob = oa + n;
-        launch_predict(x, v, xs0.as<float4>(), vin.as<float4>(), keys.as<uint32_t>(), N, c, sp,
-                       stream);
+        launch_predict(x, v, xs0.as<float4>(), vin.as<float4>(), keys.as<uint32_t>(), cell_bins(),
+                       N, c, sp, stream);
         const float4* src = xs0.as<float4>();
         const uint32_t* org_in = nullptr;
         for (int k = 0; k < I; ++k) {
@@ -896,7 +919,7 @@ struct pbf_adjoint {
             launch_search(P(t, k), s0, s0 + soa_stride(), s0 + 2 * soa_stride(), first.as<int>(), c,
                           N, NB(t, k), CN(t, k), LAM(t, k), sp, true, stream);
             launch_delta_apply(P(t, k), NB(t, k), CN(t, k), LAM(t, k), c, N, pn.as<float4>(),
-                               keys.as<uint32_t>(), sp, stream, MV(t, k),
+                               keys.as<uint32_t>(), cell_bins(), sp, stream, MV(t, k),
                                has_col() ? PRE(t, k) : nullptr);
             src = pn.as<float4>();
             org_in = org_out;
@@ -998,6 +1021,13 @@ struct pbf_adjoint {
         cuda_check(cudaGraphLaunch(it->second, stream));
     }
 
+    // Status and the cells' counts (which a failed step leaves behind).
+    void clear_status() {
+        cuda_check(cudaMemsetAsync(status.get(), 0, sizeof(unsigned), stream));
+        if (bin_count.get())
+            cuda_check(cudaMemsetAsync(bin_count.get(), 0, bin_count.bytes(), stream));
+    }
+
     void check_status() {
         unsigned h = 0;
         cuda_check(cudaMemcpyAsync(&h, status.get(), sizeof h, cudaMemcpyDeviceToHost, stream));
@@ -1022,7 +1052,7 @@ struct pbf_adjoint {
         ckpt = DeviceBuffer(static_cast<size_t>(nck) * 2 * f4b);
         steps_done = 0;
         tape_last = false;
-        cuda_check(cudaMemsetAsync(status.get(), 0, sizeof(unsigned), stream));
+        clear_status();
         cuda_check(cudaMemcpyAsync(SX(0), x0, f4b, cudaMemcpyDefault, stream));
         cuda_check(cudaMemcpyAsync(SV(0), v0, f4b, cudaMemcpyDefault, stream));
         // Before the last segment the state after t steps is in slot t % 2
@@ -1072,7 +1102,7 @@ struct pbf_adjoint {
             fail(PBF_ERR_INVALID_ARGUMENT, "null gradient pointer");
         cuda_check(cudaSetDevice(device));
         const size_t f4b = n * sizeof(float4);
-        cuda_check(cudaMemsetAsync(status.get(), 0, sizeof(unsigned), stream));
+        clear_status();
         cuda_check(cudaMemcpyAsync(gx.get(), gx_out, f4b, cudaMemcpyDefault, stream));
         cuda_check(cudaMemcpyAsync(gv.get(), gv_out, f4b, cudaMemcpyDefault, stream));
         cuda_check(cudaMemsetAsync(acc_r.get(), 0, n * sizeof(double), stream));

@@ -1,0 +1,237 @@
+// pbf_bins.cu -- the step's reorder by cell: a stable counting sort.
+//
+// A rebuild orders the particles by cell key, equal keys in their previous
+// order (src/pbf/spatial_grid.cu:188-204, a stable radix sort and the cell
+// ranges).  The keys are cell numbers, and the cell table first[] (the exclusive
+// scan of the cells' counts) is wanted in any case, so a counting sort needs
+// no digit passes:
+//   the kernel that computes a key also counts it (atomicAdd on the cell; the
+//   returned place is this particle's arrival among the cell's particles,
+//   any order);
+//   k_bin_scan          counts -> first[];
+//   k_bin_scatter       particle numbers into their cell's slots, in arrival
+//                       order (k_bin_small: both in one launch);
+//   k_bin_gather        per slot, the particle's place among its cell's ones in
+//                       their previous order (how many of the cell's numbers
+//                       are smaller), and the reorder to that place.  The
+//                       result is the stable sort's whatever the arrivals.
+// The last step reads a cell's m numbers m times; the walk that follows tests
+// at least as many pairs of each cell, so no distribution of the particles
+// makes it the larger cost.
+//
+// Bound by the latency of its dependent loads and, up to some 100,000
+// particles, by its launches (2 a rebuild up to 8,192 cells, 3 to 32,768, 4
+// above) against the radix sort's 4 to 9 small ones and the gather's search of
+// first[].  Measured on a GB300, radix sort and gather against this, five
+// rebuilds of a frame: 81 -> 64 us at 1,024 particles, 137 -> 93 at 65,536,
+// 387 -> 241 at 262,144 (two substeps), 310 -> 196 at 1,048,576, 1.67 -> 1.07
+// ms at 8,388,608.
+#include "pbf_kernels.cuh"
+
+#include <algorithm>
+
+namespace pbf {
+
+namespace {
+
+__device__ __forceinline__ bool fatal(const unsigned* status) {
+    return status != nullptr && (__ldcg(status) & kStatusFatalMask) != 0u;
+}
+
+// Exclusive scan over the block's values (one per thread); total: their sum.
+template <int THREADS>
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* warp_sums, uint32_t& total) {
+    constexpr int kWarps = THREADS / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) warp_sums[warp] = incl;
+    __syncthreads();
+    uint32_t w = lane < kWarps ? warp_sums[lane] : 0u;  // every warp scans the warps' sums
+#pragma unroll
+    for (int o = 1; o < kWarps; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += t;
+    }
+    total = __shfl_sync(0xffffffffu, w, kWarps - 1);
+    const uint32_t before = __shfl_sync(0xffffffffu, w, max(warp - 1, 0));
+    return (warp ? before : 0u) + incl - v;
+}
+
+constexpr int kItems = 8;  // cells per thread in the scans
+
+// kItems consecutive counts of the thread (0 past the last cell).  The count
+// array is padded to a multiple of kItems cells (bin_count_words).
+__device__ __forceinline__ uint32_t load_counts(const uint32_t* __restrict__ count, uint32_t at,
+                                                uint32_t cells, uint32_t (&v)[kItems]) {
+    uint32_t sum = 0u;
+#pragma unroll
+    for (int q = 0; q < kItems; q += 4) {
+        const uint4 w = at + q < cells ? __ldcg(reinterpret_cast<const uint4*>(count + at + q))
+                                       : make_uint4(0u, 0u, 0u, 0u);
+        v[q] = w.x;
+        v[q + 1] = w.y;
+        v[q + 2] = w.z;
+        v[q + 3] = w.w;
+        sum += w.x + w.y + w.z + w.w;
+    }
+    return sum;
+}
+
+// Up to kSmallCells cells: every block scans all counts into shared memory
+// (32 KB at most, from L2) and places its particles; block 0 writes first[].
+constexpr int kSmallThreads = 1024;
+constexpr uint32_t kSmallCells = kSmallThreads * kItems;
+__global__ void __launch_bounds__(kSmallThreads)
+k_bin_small(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ place,
+            const uint32_t* __restrict__ count, int n, uint32_t cells, int* __restrict__ first,
+            uint32_t* __restrict__ list, const unsigned* __restrict__ status) {
+    __shared__ uint32_t start[kSmallCells];
+    __shared__ uint32_t warp_sums[kSmallThreads / 32];
+    const int i = blockIdx.x * kSmallThreads + threadIdx.x;
+    const uint32_t key = i < n ? keys[i] : 0u, at = i < n ? place[i] : 0u;
+    uint32_t v[kItems], total;
+    const uint32_t c0 = threadIdx.x * kItems;
+    const uint32_t sum = load_counts(count, c0, cells, v);
+    if (__syncthreads_or(fatal(status))) return;
+    uint32_t run = block_scan<kSmallThreads>(sum, warp_sums, total);
+#pragma unroll
+    for (int q = 0; q < kItems; ++q) {
+        start[c0 + q] = run;
+        if (blockIdx.x == 0 && c0 + q <= cells) first[c0 + q] = static_cast<int>(run);
+        run += v[q];
+    }
+    if (blockIdx.x == 0 && cells == kSmallCells && threadIdx.x == 0)
+        first[cells] = static_cast<int>(total);
+    __syncthreads();
+    const uint32_t slot = start[key] + at;
+    if (i < n && slot < static_cast<uint32_t>(n)) list[slot] = static_cast<uint32_t>(i);
+}
+
+constexpr int kScanThreads = 512;
+constexpr uint32_t kScanTile = kScanThreads * kItems;
+// Up to this many cells the scan's blocks sum the counts before their own
+// tile themselves; above, the tiles' sums come from a launch of their own.
+constexpr uint32_t kDirectCells = 8 * kScanTile;
+
+__global__ void __launch_bounds__(kScanThreads)
+k_bin_sums(const uint32_t* __restrict__ count, uint32_t cells, uint32_t* __restrict__ sums,
+           const unsigned* __restrict__ status) {
+    __shared__ uint32_t warp_sums[kScanThreads / 32];
+    if (fatal(status)) return;
+    uint32_t v[kItems], total;
+    block_scan<kScanThreads>(
+        load_counts(count, blockIdx.x * kScanTile + threadIdx.x * kItems, cells, v), warp_sums,
+        total);
+    if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+// sums: the tiles' sums, or null (every block sums the counts before its tile).
+__global__ void __launch_bounds__(kScanThreads)
+k_bin_scan(const uint32_t* __restrict__ count, uint32_t cells, const uint32_t* __restrict__ sums,
+           int* __restrict__ first, const unsigned* __restrict__ status) {
+    __shared__ uint32_t warp_sums[2][kScanThreads / 32];
+    if (__syncthreads_or(fatal(status))) return;
+    uint32_t before = 0u;
+    if (sums) {
+        for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kScanThreads) before += sums[t];
+    } else {
+        uint32_t v[kItems];
+        for (uint32_t t = 0; t < blockIdx.x; ++t)
+            before += load_counts(count, t * kScanTile + threadIdx.x * kItems, cells, v);
+    }
+    uint32_t v[kItems], base, total;
+    const uint32_t c0 = blockIdx.x * kScanTile + threadIdx.x * kItems;
+    const uint32_t sum = load_counts(count, c0, cells, v);
+    block_scan<kScanThreads>(before, warp_sums[0], base);
+    uint32_t run = base + block_scan<kScanThreads>(sum, warp_sums[1], total);
+#pragma unroll
+    for (int q = 0; q < kItems; ++q) {
+        if (c0 + q <= cells) first[c0 + q] = static_cast<int>(run);
+        run += v[q];
+    }
+    if (c0 + kItems == cells) first[cells] = static_cast<int>(run);
+}
+
+__global__ void __launch_bounds__(kBlock)
+k_bin_scatter(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ place,
+              const int* __restrict__ first, int n, uint32_t* __restrict__ list,
+              const unsigned* __restrict__ status) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n || fatal(status)) return;
+    const uint32_t slot = static_cast<uint32_t>(__ldg(&first[keys[i]])) + place[i];
+    if (slot < static_cast<uint32_t>(n)) list[slot] = static_cast<uint32_t>(i);
+}
+
+// Thread s < n reorders the particle in slot s; thread s < cells clears the
+// count of cell s for the next rebuild.
+__global__ void __launch_bounds__(kBlock)
+k_bin_gather(const uint32_t* __restrict__ list, const uint32_t* __restrict__ keys,
+             const int* __restrict__ first, uint32_t* __restrict__ count, uint32_t cells,
+             const float4* __restrict__ xs_in, float4* __restrict__ xs_out,
+             const uint32_t* __restrict__ org_in, uint32_t* __restrict__ org_out,
+             uint32_t* __restrict__ perm, float* __restrict__ sx, float* __restrict__ sy,
+             float* __restrict__ sz, int n, const unsigned* __restrict__ status) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (fatal(status)) return;
+    if (static_cast<uint32_t>(s) < cells) count[s] = 0u;
+    if (s >= n) return;
+    const uint32_t p = list[s];
+    const uint32_t key = keys[p];
+    const float4 q = xs_in[p];
+    const uint32_t o = org_in ? org_in[p] : p;
+    const int a = __ldg(&first[key]), b = __ldg(&first[key + 1u]);
+    int dst = a;
+    for (int k = a; k < b; ++k) dst += __ldg(&list[k]) < p ? 1 : 0;
+    xs_out[dst] = q;
+    sx[dst] = q.x;
+    sy[dst] = q.y;
+    sz[dst] = q.z;
+    org_out[dst] = o;
+    if (perm) perm[dst] = p;
+}
+
+}  // namespace
+
+bool bins_apply(size_t n, uint64_t cells) {
+    return cells <= std::min<uint64_t>(8 * uint64_t(n) + 65536, uint64_t(1) << 30);
+}
+
+size_t bin_count_words(uint64_t cells) {
+    return static_cast<size_t>((cells + kItems - 1) / kItems * kItems +
+                               (cells + kScanTile - 1) / kScanTile);
+}
+
+void launch_bin_order(const CellBins& b, const uint32_t* keys, int* first, uint32_t* list, int n,
+                      uint64_t cells, const unsigned* status, cudaStream_t st) {
+    const uint32_t nc = static_cast<uint32_t>(cells);
+    if (nc <= kSmallCells) {
+        launch_k(k_bin_small, blocks_for(n, kSmallThreads), kSmallThreads, st, keys, b.place,
+                 b.count, n, nc, first, list, status);
+        return;
+    }
+    const unsigned tiles = blocks_for(nc, kScanTile);
+    uint32_t* sums = nullptr;
+    if (nc > kDirectCells) {
+        sums = b.count + (nc + kItems - 1) / kItems * kItems;
+        launch_k(k_bin_sums, tiles, kScanThreads, st, b.count, nc, sums, status);
+    }
+    launch_k(k_bin_scan, tiles, kScanThreads, st, b.count, nc, sums, first, status);
+    launch_k(k_bin_scatter, blocks_for(n), kBlock, st, keys, b.place, first, n, list, status);
+}
+
+void launch_bin_gather(const CellBins& b, const uint32_t* list, const uint32_t* keys,
+                       const int* first, uint64_t cells, const float4* xs_in, float4* xs_out,
+                       const uint32_t* org_in, uint32_t* org_out, uint32_t* perm, float* sx,
+                       float* sy, float* sz, int n, const unsigned* status, cudaStream_t st) {
+    const uint64_t threads = std::max<uint64_t>(static_cast<uint64_t>(n), cells);
+    launch_k(k_bin_gather, blocks_for(threads), kBlock, st, list, keys, first, b.count,
+             static_cast<uint32_t>(cells), xs_in, xs_out, org_in, org_out, perm, sx, sy, sz, n,
+             status);
+}
+
+}  // namespace pbf

@@ -2,10 +2,12 @@
 //
 // Hot path per constraint iteration (reference: src/pbf/pbf_solver.cu:210-258):
 //   k_predict        integrate + v_in copy + first cell keys      (integration.cu:6-32)
-//   [sort]           stable radix sort of (key, index)            (spatial_grid.cu:188-196)
-//   k_gather_first   reorder predicted positions, compose the permutation and
-//                    refresh first[] (lower bound of every cell key; the row
-//                    walk's form of cellStart/cellEnd, spatial_grid.cu:123-137)
+//   [rebuild]        stable counting sort by cell: first[] (lower bound of
+//                    every cell key; the row walk's form of cellStart/cellEnd),
+//                    reorder of the predicted positions, composed permutation
+//                    (pbf_bins.cu; spatial_grid.cu:123-196).  With far more
+//                    cells than particles a radix sort (pbf_sort.cu) and
+//                    k_gather_first.
 //   k_search<true>   neighbour walk + lambda in one pass           (neighbors.cu:3-91,
 //                                                                  pbf_solver_kernels.cu:26-105)
 //   k_delta_apply    delta p + apply + collision projection + next keys
@@ -88,14 +90,21 @@ __device__ __forceinline__ Colliders colliders_of(const StepConst& c, int i) {
     return col;
 }
 
+// The key of particle i for the next rebuild, counted in its cell.
+__device__ __forceinline__ void put_key(uint32_t* __restrict__ keys, const CellBins& bins, int i,
+                                        uint32_t key) {
+    keys[i] = key;
+    if (bins.count) bins.place[i] = atomicAdd(&bins.count[key], 1u);
+}
+
 // ---------------------------------------------------------------------------
 // integrate + collision input velocity + keys of the first rebuild
 // ---------------------------------------------------------------------------
 template <bool B>
 __global__ void __launch_bounds__(kBlock)
 k_predict(const float4* __restrict__ x, const float4* __restrict__ v, float4* __restrict__ xs,
-          float4* __restrict__ vin, uint32_t* __restrict__ keys, int n, StepConst c,
-          const unsigned* __restrict__ status) {
+          float4* __restrict__ vin, uint32_t* __restrict__ keys, CellBins bins, int n,
+          StepConst c, const unsigned* __restrict__ status) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || fatal(status)) return;
     float4 vv = v[i];
@@ -113,7 +122,7 @@ k_predict(const float4* __restrict__ x, const float4* __restrict__ v, float4* __
     GridConst g;
     uint32_t base;
     grid_of<B>(c, i, g, base);
-    keys[i] = base + key_of(g, q);
+    put_key(keys, bins, i, base + key_of(g, q));
 }
 
 __global__ void __launch_bounds__(kBlock)
@@ -955,7 +964,7 @@ template <int N, bool B, int L>
 __global__ void PBF_GATHER_REGS(48)
 k_delta_apply(const float4* __restrict__ xs, const uint32_t* __restrict__ nbr,
               const int* __restrict__ cnt, const float* __restrict__ lam, StepConst c, int n,
-              float4* __restrict__ xs_out, uint32_t* __restrict__ keys_out,
+              float4* __restrict__ xs_out, uint32_t* __restrict__ keys_out, CellBins bins,
               uint8_t* __restrict__ moved, float4* __restrict__ pre,
               unsigned* __restrict__ status) {
     int i, sub;
@@ -987,7 +996,7 @@ k_delta_apply(const float4* __restrict__ xs, const uint32_t* __restrict__ nbr,
         GridConst g;
         uint32_t base;
         grid_of<B>(c, i, g, base);
-        keys_out[i] = base + key_of(g, q);
+        put_key(keys_out, bins, i, base + key_of(g, q));
     }
 }
 
@@ -1452,11 +1461,10 @@ k_integrate(const float4* __restrict__ x, float4* __restrict__ xs, float4* __res
 
 // --- launchers ---------------------------------------------------------------
 void launch_predict(const float4* x, const float4* v, float4* xs, float4* vin, uint32_t* keys,
-                    int n, const StepConst& c, const unsigned* status, cudaStream_t st) {
-    if (c.scenes)
-        launch_k(k_predict<true>, blocks_for(n), kBlock, st, x, v, xs, vin, keys, n, c, status);
-    else
-        launch_k(k_predict<false>, blocks_for(n), kBlock, st, x, v, xs, vin, keys, n, c, status);
+                    const CellBins& bins, int n, const StepConst& c, const unsigned* status,
+                    cudaStream_t st) {
+    launch_k(c.scenes ? k_predict<true> : k_predict<false>, blocks_for(n), kBlock, st, x, v, xs,
+             vin, keys, bins, n, c, status);
 }
 void launch_cell_ranges(const uint32_t* skeys, int* cs, int* ce, int n, const unsigned* status,
                         cudaStream_t st) {
@@ -1624,7 +1632,8 @@ void launch_nb_scan(const int* cnt, uint32_t* off, size_t cap, int n, uint32_t* 
 template <bool B>
 void launch_delta_apply_b(const float4* xs, const uint32_t* nbr, const int* cnt, const float* lam,
                           const StepConst& c, int n, float4* xs_out, uint32_t* keys_out,
-                          uint8_t* moved, float4* pre, unsigned* status, cudaStream_t st) {
+                          const CellBins& bins, uint8_t* moved, float4* pre, unsigned* status,
+                          cudaStream_t st) {
     const int bs = tuned_block(c, kTunedDelta);
     const unsigned g = blocks_for(n, bs);
     const int L = split_lanes(c, n);
@@ -1632,16 +1641,16 @@ void launch_delta_apply_b(const float4* xs, const uint32_t* nbr, const int* cnt,
 #define PBF_DELTA_CASE(N)                                                                        \
     if (L == 8)                                                                                  \
         launch_k(k_delta_apply<N, B, 8>, gl, bs, st, xs, nbr, cnt, lam, c, n, xs_out, keys_out,  \
-                 moved, pre, status);                                                            \
+                 bins, moved, pre, status);                                                            \
     else if (L == 4)                                                                             \
         launch_k(k_delta_apply<N, B, 4>, gl, bs, st, xs, nbr, cnt, lam, c, n, xs_out, keys_out,  \
-                 moved, pre, status);                                                            \
+                 bins, moved, pre, status);                                                            \
     else if (L == 2)                                                                             \
         launch_k(k_delta_apply<N, B, 2>, gl, bs, st, xs, nbr, cnt, lam, c, n, xs_out, keys_out,  \
-                 moved, pre, status);                                                            \
+                 bins, moved, pre, status);                                                            \
     else                                                                                         \
         launch_k(k_delta_apply<N, B, 1>, g, bs, st, xs, nbr, cnt, lam, c, n, xs_out, keys_out,   \
-                 moved, pre, status)
+                 bins, moved, pre, status)
     switch (c.sc.k != 0.0f ? c.sc.n : 0) {
         case 1: PBF_DELTA_CASE(1); break;
         case 2: PBF_DELTA_CASE(2); break;
@@ -1653,13 +1662,14 @@ void launch_delta_apply_b(const float4* xs, const uint32_t* nbr, const int* cnt,
 }
 void launch_delta_apply(const float4* xs, const uint32_t* nbr, const int* cnt, const float* lam,
                         const StepConst& c, int n, float4* xs_out, uint32_t* keys_out,
-                        unsigned* status, cudaStream_t st, uint8_t* moved, float4* pre) {
+                        const CellBins& bins, unsigned* status, cudaStream_t st, uint8_t* moved,
+                        float4* pre) {
     if (c.scenes)
-        launch_delta_apply_b<true>(xs, nbr, cnt, lam, c, n, xs_out, keys_out, moved, pre, status,
-                                   st);
+        launch_delta_apply_b<true>(xs, nbr, cnt, lam, c, n, xs_out, keys_out, bins, moved, pre,
+                                   status, st);
     else
-        launch_delta_apply_b<false>(xs, nbr, cnt, lam, c, n, xs_out, keys_out, moved, pre, status,
-                                    st);
+        launch_delta_apply_b<false>(xs, nbr, cnt, lam, c, n, xs_out, keys_out, bins, moved, pre,
+                                    status, st);
 }
 void launch_finalize(const uint32_t* org, const float4* x_old, const float4* vin_old,
                      const float4* v_old, const uint32_t* id_old, const float4* xs, int n,

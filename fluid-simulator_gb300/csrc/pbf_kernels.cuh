@@ -92,9 +92,17 @@ inline void launch_k(void (*k)(P...), unsigned grid, unsigned block, cudaStream_
     launch_error_check(cudaLaunchKernelEx(&cfg, k, static_cast<P>(a)...));
 }
 
+// Counting-sort state of one solver (pbf_bins.cu): count[cell] (zero between
+// rebuilds) and every particle's place among its cell's arrivals, written with
+// the keys.  count null: keys only.
+struct CellBins {
+    uint32_t* count = nullptr;
+    uint32_t* place = nullptr;
+};
+
 // --- step kernels (pbf_kernels.cu) -----------------------------------------
 void launch_predict(const float4* x, const float4* v, float4* xs, float4* vin, uint32_t* keys,
-                    int n, const StepConst& c, const unsigned* status, cudaStream_t st);
+                    const CellBins& bins, int n, const StepConst& c, const unsigned* status, cudaStream_t st);
 void launch_cell_ranges(const uint32_t* skeys, int* cell_start, int* cell_end, int n,
                         const unsigned* status, cudaStream_t st);
 // Reorders predicted positions (float4 and x/y/z component arrays for the
@@ -123,7 +131,8 @@ void launch_search_xsph(const float4* xs, const float* sx, const float* sy, cons
 // the projection.
 void launch_delta_apply(const float4* xs, const uint32_t* nbr, const int* cnt, const float* lam,
                         const StepConst& c, int n, float4* xs_out, uint32_t* keys_out,
-                        unsigned* status, cudaStream_t st, uint8_t* moved = nullptr,
+                        const CellBins& bins, unsigned* status, cudaStream_t st,
+                        uint8_t* moved = nullptr,
                         float4* pre = nullptr);
 // Compact lists: neighbour counts of the walk (no list written), then the
 // exclusive scan of the counts into off (n + 1 entries; a total above cap
@@ -171,6 +180,21 @@ void launch_collide(float4* pos, int n, const StepConst& c, int kind, unsigned* 
                     cudaStream_t st);
 void launch_integrate(const float4* x, float4* xs, float4* v, int n, const StepConst& c,
                       cudaStream_t st);
+
+// --- counting sort by cell (pbf_bins.cu) -------------------------------------
+// Whether the step's rebuilds use it: cells in proportion to the particles.
+bool bins_apply(size_t n, uint64_t cells);
+size_t bin_count_words(uint64_t cells);  // of CellBins::count, zeroed once
+// From keys and their counts: the cell table first[] (cells + 1 entries) and
+// the particle numbers cell by cell, in arrival order.
+void launch_bin_order(const CellBins& b, const uint32_t* keys, int* first, uint32_t* list, int n,
+                      uint64_t cells, const unsigned* status, cudaStream_t st);
+// The reorder (as launch_gather_first; perm, optional: slot -> previous slot),
+// equal keys in their previous order; clears the counts.
+void launch_bin_gather(const CellBins& b, const uint32_t* list, const uint32_t* keys,
+                       const int* first, uint64_t cells, const float4* xs_in, float4* xs_out,
+                       const uint32_t* org_in, uint32_t* org_out, uint32_t* perm, float* sx,
+                       float* sy, float* sz, int n, const unsigned* status, cudaStream_t st);
 
 // --- stable LSD radix sort of (key, index) pairs (pbf_sort.cu) ---------------
 struct SortPlan {

@@ -213,6 +213,11 @@ struct pbf_solver {
     DeviceBuffer f4[kF4Pool];
     DeviceBuffer ids[2], org[2];
     DeviceBuffer keys, skeys, sidx, akeys, aidx;
+    // Counting sort (bins): the cells' counts, zero between rebuilds except
+    // after a failed or unchecked run; akeys holds the arrival places and
+    // aidx the lists.
+    DeviceBuffer bin_count;
+    bool bins_dirty = true;
     DeviceBuffer cell_first, nbr, cnt, lam, sort_scratch, status, tmp4, ftmp;
     DeviceBuffer soa;  // x, y, z components of the reordered predicted positions
     // Component array stride (see soa_stride_for).
@@ -324,6 +329,24 @@ struct pbf_solver {
         clear_graphs();
     }
 
+    // The counting sort's state when the rebuilds of n particles use it.
+    CellBins cell_bins() const {
+        CellBins b;
+        if (bin_count.get() && bins_apply(n, cells)) {
+            b.count = bin_count.as<uint32_t>();
+            b.place = akeys.as<uint32_t>();
+        }
+        return b;
+    }
+    // Before the first frame of a run: status and, unless the last run is
+    // known to have ended well, the counts.
+    void clear_status() {
+        cuda_check(cudaMemsetAsync(status.get(), 0, sizeof(unsigned), stream));
+        if (bins_dirty && bin_count.get())
+            cuda_check(cudaMemsetAsync(bin_count.get(), 0, bin_count.bytes(), stream));
+        bins_dirty = true;  // until check_status
+    }
+
     // ---- frame emission -----------------------------------------------------
     // Enqueues one frame on `st` starting from roles (ix, iv, iid) and returns
     // the roles after it.  Buffer roles are handed out lowest-free-first, so
@@ -346,6 +369,7 @@ struct pbf_solver {
         auto give = [&](int i) { used[i] = false; };
         auto P = [&](int i) { return f4[i].as<float4>(); };
         const SortPlan plan = make_sort_plan(N, cells, sort_tile);
+        const CellBins bins = cell_bins();
         const bool post = prm.xsphViscosity != 0.0f || prm.vorticityStrength != 0.0f;
 
         auto M = [&](int stage) {
@@ -355,22 +379,35 @@ struct pbf_solver {
             const int xs0 = take();
             const int vin = take();
             M(kStPredict);
-            launch_predict(P(rx), P(rv), P(xs0), P(vin), keys.as<uint32_t>(), N, c, sp, st);
+            launch_predict(P(rx), P(rv), P(xs0), P(vin), keys.as<uint32_t>(), bins, N, c, sp, st);
             int cur = xs0;
             int org_cur = -1;
             auto rebuild = [&]() {
                 M(kStSort);
-                launch_sort(plan, keys.as<uint32_t>(), skeys.as<uint32_t>(), sidx.as<uint32_t>(),
-                            akeys.as<uint32_t>(), aidx.as<uint32_t>(), sort_scratch.get(), sp, st);
+                if (bins.count)
+                    launch_bin_order(bins, keys.as<uint32_t>(), cell_first.as<int>(),
+                                     aidx.as<uint32_t>(), N, cells, sp, st);
+                else
+                    launch_sort(plan, keys.as<uint32_t>(), skeys.as<uint32_t>(),
+                                sidx.as<uint32_t>(), akeys.as<uint32_t>(), aidx.as<uint32_t>(),
+                                sort_scratch.get(), sp, st);
                 const int nxt = take();
                 const int org_next = org_cur < 0 ? 0 : 1 - org_cur;
                 M(kStGatherRanges);
-                launch_gather_first(sidx.as<uint32_t>(), P(cur), P(nxt),
-                                    org_cur < 0 ? nullptr : org[org_cur].as<uint32_t>(),
-                                    org[org_next].as<uint32_t>(), soa.as<float>(),
-                                    soa.as<float>() + soa_stride(),
-                                    soa.as<float>() + 2 * soa_stride(), N, skeys.as<uint32_t>(),
-                                    cells, cell_first.as<int>(), sp, st);
+                if (bins.count)
+                    launch_bin_gather(bins, aidx.as<uint32_t>(), keys.as<uint32_t>(),
+                                      cell_first.as<int>(), cells, P(cur), P(nxt),
+                                      org_cur < 0 ? nullptr : org[org_cur].as<uint32_t>(),
+                                      org[org_next].as<uint32_t>(), nullptr, soa.as<float>(),
+                                      soa.as<float>() + soa_stride(),
+                                      soa.as<float>() + 2 * soa_stride(), N, sp, st);
+                else
+                    launch_gather_first(sidx.as<uint32_t>(), P(cur), P(nxt),
+                                        org_cur < 0 ? nullptr : org[org_cur].as<uint32_t>(),
+                                        org[org_next].as<uint32_t>(), soa.as<float>(),
+                                        soa.as<float>() + soa_stride(),
+                                        soa.as<float>() + 2 * soa_stride(), N,
+                                        skeys.as<uint32_t>(), cells, cell_first.as<int>(), sp, st);
                 give(cur);
                 cur = nxt;
                 org_cur = org_next;
@@ -394,8 +431,11 @@ struct pbf_solver {
                               nbr.as<uint32_t>(), cnt.as<int>(), lam.as<float>(), sp, true, st);
                 const int nxt = take();
                 M(kStDeltaApply);
+                // Without the final rebuild nothing uses the last keys.
+                const bool last = it + 1 == prm.solverIterations && !post;
                 launch_delta_apply(P(cur), nbr.as<uint32_t>(), cnt.as<int>(), lam.as<float>(), c,
-                                   N, P(nxt), keys.as<uint32_t>(), sp, st);
+                                   N, P(nxt), keys.as<uint32_t>(), last ? CellBins{} : bins, sp,
+                                   st);
                 give(cur);
                 cur = nxt;
             }
@@ -518,7 +558,7 @@ struct pbf_solver {
         use_device();
         if (n == 0) fail(PBF_ERR_LOGIC, "no particles to profile");
         upload_colliders();
-        cuda_check(cudaMemsetAsync(status.get(), 0, sizeof(unsigned), stream));
+        clear_status();
         auto& g = graph_for(ix, iv, iid, true);
         cuda_check(cudaGraphLaunch(g.first, stream));
         std::tie(ix, iv, iid) = g.second;
@@ -648,13 +688,14 @@ struct pbf_solver {
         if (s & kStatusNotConverged) fail(PBF_ERR_RUNTIME, "Collision constraints did not converge");
         if (s & kStatusListOverflow)
             fail(PBF_ERR_OVERFLOW, "Neighbor lists exceed the compact list capacity");
+        bins_dirty = false;
     }
 
     void run_frames(size_t frames, bool sync) {
         use_device();
         if (n == 0 || frames == 0) return;
         upload_colliders();
-        cuda_check(cudaMemsetAsync(status.get(), 0, sizeof(unsigned), stream));
+        clear_status();
         enqueue_frames(frames);
         if (sync) check_status();
     }
@@ -707,6 +748,9 @@ struct pbf_solver {
         for (auto& b : nids) b.allocate(u4b);
         for (auto& b : norg) b.allocate(u4b);
         DeviceBuffer nkeys(u4b), nskeys(u4b), nsidx(u4b), nakeys(u4b), naidx(u4b);
+        DeviceBuffer nbins;
+        if (bins_apply(max_particles, ncells))
+            nbins.allocate(bin_count_words(ncells) * sizeof(uint32_t));
         DeviceBuffer nfirst((ncells + 1) * sizeof(int));
         DeviceBuffer nsoa(3 * soa_stride_for(max_particles) * sizeof(float));
         DeviceBuffer nnbr((lcap > 0 ? lcap : strd * size_t(maxnb)) * sizeof(uint32_t));
@@ -729,6 +773,9 @@ struct pbf_solver {
         sidx = std::move(nsidx);
         akeys = std::move(nakeys);
         aidx = std::move(naidx);
+        bin_count = std::move(nbins);
+        bins_dirty = true;
+        cuda_check(cudaMemsetAsync(aidx.get(), 0, u4b, stream));
         cell_first = std::move(nfirst);
         soa = std::move(nsoa);
         nbr = std::move(nnbr);
