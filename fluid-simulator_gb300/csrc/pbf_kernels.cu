@@ -26,8 +26,7 @@
 #include "pbf_kernels.cuh"
 
 #include "pbf_common.h"
-
-#include <math_constants.h>
+#include "pbf_device.cuh"
 
 #include <algorithm>
 
@@ -43,59 +42,6 @@ void launch_error_check(cudaError_t e) { cuda_check(e); }
 
 
 namespace {
-
-__device__ __forceinline__ bool fatal(const unsigned* status) {
-    return status != nullptr && (__ldcg(status) & kStatusFatalMask) != 0u;
-}
-
-// The scene of particle slot i in a batched solver.
-__device__ __forceinline__ const SceneConst& scene_of(const StepConst& c, int i) {
-    return c.scenes[__ldg(&c.sid[i])];
-}
-
-// First entry and entry stride of particle i's neighbour list.
-__device__ __forceinline__ size_t nb_first(const StepConst& c, int i) {
-    return c.nb_off ? static_cast<size_t>(__ldg(&c.nb_off[i])) : static_cast<size_t>(i);
-}
-__device__ __forceinline__ size_t nb_step(const StepConst& c) {
-    return c.nb_off ? size_t(1) : c.stride;
-}
-
-// Grid and first global cell key of slot i: the scene's (B) or c.g.
-template <bool B>
-__device__ __forceinline__ void grid_of(const StepConst& c, int i, GridConst& g, uint32_t& base) {
-    if constexpr (B) {
-        const SceneConst& s = scene_of(c, i);
-        g = s.g;
-        base = s.cell_base;
-    } else {
-        g = c.g;
-        base = 0u;
-    }
-}
-
-// Colliders with the container of slot i's scene (B) or c.col.
-template <bool B>
-__device__ __forceinline__ Colliders colliders_of(const StepConst& c, int i) {
-    Colliders col = c.col;
-    if constexpr (B) {
-        const SceneConst& s = scene_of(c, i);
-        col.cminx = s.cminx;
-        col.cminy = s.cminy;
-        col.cminz = s.cminz;
-        col.cmaxx = s.cmaxx;
-        col.cmaxy = s.cmaxy;
-        col.cmaxz = s.cmaxz;
-    }
-    return col;
-}
-
-// The key of particle i for the next rebuild, counted in its cell.
-__device__ __forceinline__ void put_key(uint32_t* __restrict__ keys, const CellBins& bins, int i,
-                                        uint32_t key) {
-    keys[i] = key;
-    if (bins.count) bins.place[i] = atomicAdd(&bins.count[key], 1u);
-}
 
 // ---------------------------------------------------------------------------
 // integrate + collision input velocity + keys of the first rebuild
@@ -227,21 +173,6 @@ k_gather_first(const uint32_t* __restrict__ perm, const float4* __restrict__ xs_
 // (src/pbf/neighbors.cu:52-86).  With LAMBDA the constraint terms of
 // computeLambda are accumulated in that same list order.
 // ---------------------------------------------------------------------------
-struct LambdaAcc {
-    float wsum, s2, gx, gy, gz;
-};
-
-__device__ __forceinline__ void lambda_add(const KernelConst& k, LambdaAcc& a, float dx, float dy,
-                                           float dz, float d2) {
-    a.wsum = fadd(a.wsum, poly6(k, d2));
-    float gx, gy, gz;
-    spiky(k, dx, dy, dz, d2, gx, gy, gz);
-    a.s2 = ffma(gz, gz, ffma(gy, gy, ffma(gx, gx, a.s2)));
-    a.gx = fadd(a.gx, gx);
-    a.gy = fadd(a.gy, gy);
-    a.gz = fadd(a.gz, gz);
-}
-
 // Two neighbours' terms, lane 0 first: the same sums as two lambda_add calls.
 __device__ __forceinline__ void lambda_add2(const KernelConst& k, LambdaAcc& a, f32x2 dx, f32x2 dy,
                                             f32x2 dz, f32x2 d2) {
@@ -258,97 +189,6 @@ __device__ __forceinline__ void lambda_add2(const KernelConst& k, LambdaAcc& a, 
     a.gy = fadd(fadd(a.gy, y0), y1);
     a.gz = fadd(fadd(a.gz, z0), z1);
 }
-
-__device__ __forceinline__ float lambda_finish(float mass, float rho0, float gs2, float eps,
-                                               const LambdaAcc& a) {
-    const float rho = fmul(mass, a.wsum);
-    const float g2 = dist2(a.gx, a.gy, a.gz);
-    const float denom = ffma(gs2, fadd(a.s2, g2), eps);
-    const float C = fsub(fdiv(rho, rho0), 1.0f);
-    return fdiv(-C, denom);
-}
-__device__ __forceinline__ float lambda_finish(const StepConst& c, const LambdaAcc& a) {
-    return lambda_finish(c.mass, c.rho0, c.gs2, c.lambda_eps, a);
-}
-
-// Squared distances from coordinate p to the slabs of the cells below and
-// above cell k on one axis (cell k spans [lo + k cell, lo + (k + 1) cell);
-// the clamped end cells extend to infinity, which changes neither distance),
-// each first reduced by eps.  Margin arithmetic only: it decides which cells
-// the walk reads, never a neighbour.
-__device__ __forceinline__ void slab_dist2(float p, float lo, float cell, int k, float eps,
-                                           float& below, float& above) {
-    const float b0 = fmaf(static_cast<float>(k), cell, lo);
-    const float b1 = fmaf(static_cast<float>(k + 1), cell, lo);
-    const float d0 = fmaxf(p - b0 - eps, 0.0f);
-    const float d1 = fmaxf(b1 - p - eps, 0.0f);
-    below = d0 * d0;
-    above = d1 * d1;
-}
-
-// The neighbour walk of particle i (position pi): writes the list slot-major
-// at out[slot * stride] (at most cap entries) and returns the full count.
-// STORE = false counts the hits without writing the list.
-// The stencil rows of particle i, as the walks visit them: z0..z1 x y0..y1
-// (clamped to the grid), and range(z, y) gives row (z, y)'s candidate index
-// range [s, e): its cells x0..x1 are consecutive keys.  Keys fit in 32 bits
-// (cells < 2^32 is checked at initialisation), so the reference's 64-bit key
-// arithmetic truncates to the same values.
-// Cell pruning (radius 1): a stencil cell whose box lies farther than h
-// from the particle holds no neighbour, so range() returns false for the
-// rows (y, z) that far and leaves out the end cells of a row that far.  Per
-// axis, eps = 2^-14 (|p| + |min| + cell) covers the FP32 rounding of every
-// cell index (floor((p - min) / cell)) and of the candidates' differences,
-// and the bound h2 (1 + 2^-10) the rounding of d2: only certain misses are
-// left out, so the list is entry for entry the unpruned walk's.
-template <bool B>
-struct StencilRows {
-    GridConst g;
-    uint32_t base, gx, gxy;
-    int cx, cy, cz, x0, x1, y0, y1, z0, z1;
-    bool prune;
-    float xb2, xa2, yb2, ya2, zb2, za2, lim2;
-    __device__ __forceinline__ StencilRows(const StepConst& c, int i, float4 pi) {
-        grid_of<B>(c, i, g, base);
-        cell_of(g, pi.x, pi.y, pi.z, cx, cy, cz);
-        const int R = g.radius;
-        x0 = max(0, cx - R);
-        x1 = min(g.gx - 1, cx + R);
-        y0 = max(0, cy - R);
-        y1 = min(g.gy - 1, cy + R);
-        z0 = max(0, cz - R);
-        z1 = min(g.gz - 1, cz + R);
-        gx = static_cast<uint32_t>(g.gx);
-        gxy = gx * static_cast<uint32_t>(g.gy);
-        prune = c.prune_cells && R == 1;
-        xb2 = xa2 = yb2 = ya2 = zb2 = za2 = lim2 = 0.0f;
-        if (prune) {
-            const float eps = 6.103515625e-05f *
-                              (fabsf(pi.x) + fabsf(pi.y) + fabsf(pi.z) + fabsf(g.minx) +
-                               fabsf(g.miny) + fabsf(g.minz) + g.cell);
-            slab_dist2(pi.x, g.minx, g.cell, cx, eps, xb2, xa2);
-            slab_dist2(pi.y, g.miny, g.cell, cy, eps, yb2, ya2);
-            slab_dist2(pi.z, g.minz, g.cell, cz, eps, zb2, za2);
-            lim2 = c.k.h2 * 1.0009765625f;
-        }
-    }
-    __device__ __forceinline__ bool range(const int* __restrict__ first, int z, int y, int& s,
-                                          int& e) const {
-        int xa = x0, xb = x1;
-        if (prune) {
-            const float dyz = (z < cz ? zb2 : (z > cz ? za2 : 0.0f)) +
-                              (y < cy ? yb2 : (y > cy ? ya2 : 0.0f));
-            if (dyz > lim2) return false;
-            if (xa < cx && dyz + xb2 > lim2) xa = cx;
-            if (xb > cx && dyz + xa2 > lim2) xb = cx;
-        }
-        const uint32_t row =
-            base + static_cast<uint32_t>(y) * gx + static_cast<uint32_t>(z) * gxy;
-        s = __ldg(&first[row + static_cast<uint32_t>(xa)]);
-        e = __ldg(&first[row + static_cast<uint32_t>(xb) + 1u]);
-        return true;
-    }
-};
 
 // Bits of a 32-candidate chunk from j0 that belong to the row range [s, e),
 // less the particle i itself.
@@ -471,12 +311,7 @@ __device__ __forceinline__ float lambda_of_list(const StepConst& c, int i, float
         const float dx = fsub(pi.x, pj.x), dy = fsub(pi.y, pj.y), dz = fsub(pi.z, pj.z);
         lambda_add(c.k, acc, dx, dy, dz, dist2(dx, dy, dz));
     }
-    if constexpr (B) {
-        const SceneConst& sc = scene_of(c, i);
-        return lambda_finish(sc.mass, sc.rho0, sc.gs2, c.lambda_eps, acc);
-    } else {
-        return lambda_finish(c, acc);
-    }
+    return lambda_of_acc<B>(c, i, acc);
 }
 
 // What k_search does once particle i's list (count entries) is written.
@@ -505,170 +340,6 @@ k_search(const float4* __restrict__ xs, const float* __restrict__ sx,
     uint32_t* __restrict__ out = nbr + nb_first(c, i);
     const int count = walk<B>(c, i, pi, sx, sy, sz, first, out, c.max_nb);
     search_tail<LAMBDA, B>(c, i, pi, xs, out, count, cnt, lam, status);
-}
-
-// The walk on a group of L lanes (gmask; lane `sub`), for scenes too small
-// to fill the GPU with one thread per particle.  The lanes visit the same
-// rows and chunks together; lane q tests candidates [qW, (q + 1)W) of each
-// 32-candidate chunk (W = 32 / L), the group ORs the hit masks, and each
-// lane writes its own hits at their places in the list (the hits of lower
-// lanes first).  The list is walk()'s, entry for entry; the count is
-// returned on every lane.
-template <bool B, int L>
-__device__ __forceinline__ int walk_chunks(const StepConst& c, int i, int sub, unsigned gmask,
-                                           float4 pi, const float* __restrict__ sx,
-                                           const float* __restrict__ sy,
-                                           const float* __restrict__ sz,
-                                           const int* __restrict__ first,
-                                           uint32_t* __restrict__ out) {
-    constexpr int W = 32 / L;
-    const StencilRows<B> rows(c, i, pi);
-    const f32x2 h2u = splat2(__uint_as_float(__float_as_uint(c.k.h2) + 1u));
-    const size_t stride = nb_step(c);
-    const int cap = c.max_nb;
-    const f32x2 px = splat2(pi.x), py = splat2(pi.y), pz = splat2(pi.z);
-    const uint32_t lower = (1u << (sub * W)) - 1u;  // bits of lower lanes' candidates
-    const uint32_t own = W == 32 ? 0xffffffffu : (((1u << W) - 1u) << (sub * W));
-    int count = 0;
-    for (int z = rows.z0; z <= rows.z1; ++z)
-        for (int y = rows.y0; y <= rows.y1; ++y) {
-            int s, e;
-            if (!rows.range(first, z, y, s, e)) continue;
-            for (int j0 = s & ~3; j0 < e; j0 += 32) {
-                const int jb = j0 + sub * W;
-                uint32_t acc = 0u;
-                if (jb < e) {
-#pragma unroll
-                    for (int q = 0; q < W; q += 4) {
-                        const float4 X = __ldg(reinterpret_cast<const float4*>(sx + jb + q));
-                        const float4 Y = __ldg(reinterpret_cast<const float4*>(sy + jb + q));
-                        const float4 Z = __ldg(reinterpret_cast<const float4*>(sz + jb + q));
-                        const f32x2 da = dist2x2(sub2(px, pack2(X.x, X.y)),
-                                                 sub2(py, pack2(Y.x, Y.y)),
-                                                 sub2(pz, pack2(Z.x, Z.y)));
-                        const f32x2 db = dist2x2(sub2(px, pack2(X.z, X.w)),
-                                                 sub2(py, pack2(Y.z, Y.w)),
-                                                 sub2(pz, pack2(Z.z, Z.w)));
-                        float a0, a1, b0, b1;
-                        unpack2(sub2(da, h2u), a0, a1);
-                        unpack2(sub2(db, h2u), b0, b1);
-                        acc = __funnelshift_l(__float_as_uint(a0), acc, 1);
-                        acc = __funnelshift_l(__float_as_uint(a1), acc, 1);
-                        acc = __funnelshift_l(__float_as_uint(b0), acc, 1);
-                        acc = __funnelshift_l(__float_as_uint(b1), acc, 1);
-                    }
-                }
-                // This lane's W hit bits at its place in the chunk's mask.
-                uint32_t mask = (W == 32 ? __brev(acc) : (__brev(acc) >> (32 - W))) << (sub * W);
-#pragma unroll
-                for (int d = 1; d < L; d <<= 1) mask |= __shfl_xor_sync(gmask, mask, d, L);
-                mask &= chunk_valid(j0, s, e, i);
-                uint32_t mine = mask & own;
-                int pos = count + __popc(mask & lower);
-                while (mine) {
-                    const int b = __ffs(mine) - 1;
-                    mine &= mine - 1u;
-                    if (pos < cap) out[static_cast<size_t>(pos) * stride] = static_cast<uint32_t>(j0 + b);
-                    ++pos;
-                }
-                count += __popc(mask);
-            }
-        }
-    __syncwarp(gmask);  // the group's stores ordered before any lane reads the list
-    return count;
-}
-
-
-template <int L>
-__device__ __forceinline__ unsigned lane_group_mask() {
-    const unsigned lane = threadIdx.x & 31u;
-    return ((1u << L) - 1u) << (lane & ~(L - 1u));
-}
-
-// A neighbour sum of particle i spread over its group of L lanes (gmask),
-// the accumulation kept on lane 0 in list order.  In round m, lane q
-// evaluates the V terms of list entry mL + q (term(k, t)), the group hands
-// them to lane 0 by shuffles, and lane 0 adds them in entry order
-// (add(u)).  Each term is the value one lane computes for that entry alone
-// and the additions run in the same order, so the sum is the one-lane
-// loop's, bit for bit; the lanes share the gathers and the term arithmetic.
-template <int L, int V, class Term, class Add>
-__device__ __forceinline__ void group_sum(int count, int sub, unsigned gmask, Term term, Add add) {
-    for (int k0 = 0; k0 < count; k0 += L) {
-        float t[V];
-#pragma unroll
-        for (int v = 0; v < V; ++v) t[v] = 0.0f;
-        if (k0 + sub < count) term(k0 + sub, t);
-#pragma unroll
-        for (int q = 0; q < L; ++q) {
-            float u[V];
-#pragma unroll
-            for (int v = 0; v < V; ++v) u[v] = __shfl_sync(gmask, t[v], q, L);
-            if (sub == 0 && k0 + q < count) add(u);
-        }
-    }
-}
-
-// lambda_of_list on a group of L lanes (the value is lane 0's).
-template <bool B, int L>
-__device__ __forceinline__ float lambda_group(const StepConst& c, int i, int sub, unsigned gmask,
-                                              float4 pi, const float4* __restrict__ xs,
-                                              const uint32_t* __restrict__ out, size_t stride,
-                                              int count) {
-    LambdaAcc acc{c.k.c_poly6, 0.0f, 0.0f, 0.0f, 0.0f};
-    group_sum<L, 4>(
-        count, sub, gmask,
-        [&](int k, float (&t)[4]) {
-            const float4 pj = __ldg(&xs[out[static_cast<size_t>(k) * stride]]);
-            const float dx = fsub(pi.x, pj.x), dy = fsub(pi.y, pj.y), dz = fsub(pi.z, pj.z);
-            const float d2 = dist2(dx, dy, dz);
-            t[0] = poly6(c.k, d2);
-            spiky(c.k, dx, dy, dz, d2, t[1], t[2], t[3]);
-        },
-        [&](const float (&u)[4]) {
-            acc.wsum = fadd(acc.wsum, u[0]);
-            acc.s2 = ffma(u[3], u[3], ffma(u[2], u[2], ffma(u[1], u[1], acc.s2)));
-            acc.gx = fadd(acc.gx, u[1]);
-            acc.gy = fadd(acc.gy, u[2]);
-            acc.gz = fadd(acc.gz, u[3]);
-        });
-    if constexpr (B) {
-        const SceneConst& sc = scene_of(c, i);
-        return lambda_finish(sc.mass, sc.rho0, sc.gs2, c.lambda_eps, acc);
-    } else {
-        return lambda_finish(c, acc);
-    }
-}
-
-// k_search with L lanes per particle (slot-major lists only): the group
-// walks the rows together (walk_chunks) and shares lambda's neighbour terms
-// (lambda_group).  For scenes too small to fill the GPU with one thread per
-// particle, where a walk is bound by the latency of one thread's row after
-// row.
-template <bool LAMBDA, bool B, int L>
-__global__ void __launch_bounds__(kMaxTunedBlock)
-k_search_split(const float4* __restrict__ xs, const float* __restrict__ sx,
-               const float* __restrict__ sy, const float* __restrict__ sz,
-               const int* __restrict__ first, StepConst c, int n, uint32_t* __restrict__ nbr,
-               int* __restrict__ cnt, float* __restrict__ lam, unsigned* __restrict__ status) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = t / L, sub = t % L;
-    if (i >= n) return;  // whole groups
-    const unsigned gmask = lane_group_mask<L>();
-    if (__any_sync(gmask, fatal(status))) return;
-    const float4 pi = xs[i];
-    uint32_t* __restrict__ out = nbr + nb_first(c, i);
-    const int count = walk_chunks<B, L>(c, i, sub, gmask, pi, sx, sy, sz, first, out);
-    if (sub == 0) {
-        cnt[i] = count;
-        if (count > c.max_nb) atomicOr(status, kStatusNeighborOverflow);
-    }
-    if (LAMBDA) {
-        const float l = count > c.max_nb
-                            ? CUDART_NAN_F
-                            : lambda_group<B, L>(c, i, sub, gmask, pi, xs, out, nb_step(c), count);
-        if (sub == 0) lam[i] = l;
-    }
 }
 
 // Compact lists, first pass: the walk's neighbour count only.
@@ -778,10 +449,6 @@ k_nb_scan_add(int n, size_t cap, const unsigned long long* __restrict__ tile_sum
         off[n] = static_cast<uint32_t>(min(total, 0xffffffffull));
         if (total > cap) atomicOr(status, kStatusListOverflow);
     }
-}
-
-__device__ __forceinline__ bool count_ok(int count, int max_nb) {
-    return count >= 0 && count <= max_nb;
 }
 
 // Walks a slot-major list in order, four neighbours at a time: their four
@@ -903,73 +570,18 @@ __device__ __forceinline__ void delta_sum(const StepConst& c, const float4* __re
     dpz = fmul(gs, az);
 }
 
-// delta_sum with its terms spread over a group of L lanes (lane 0's value).
-template <int N, int L>
-__device__ __forceinline__ void delta_sum_group(const StepConst& c, const float4* __restrict__ xs,
-                                                const uint32_t* __restrict__ nbr,
-                                                const float* __restrict__ lam, int i, int sub,
-                                                unsigned gmask, int count, float4 pi, float gs,
-                                                float& dpx, float& dpy, float& dpz) {
-    const float li = lam[i];
-    const uint32_t* row = nbr + nb_first(c, i);
-    const size_t st = nb_step(c);
-    float ax = 0.0f, ay = 0.0f, az = 0.0f;
-    group_sum<L, 4>(
-        count, sub, gmask,
-        [&](int k, float (&t)[4]) {
-            const uint32_t j = __ldg(&row[static_cast<size_t>(k) * st]);
-            const float4 pj = __ldg(&xs[j]);
-            const float lj = __ldg(&lam[j]);
-            const float dx = fsub(pi.x, pj.x), dy = fsub(pi.y, pj.y), dz = fsub(pi.z, pj.z);
-            const float d2 = dist2(dx, dy, dz);
-            spiky(c.k, dx, dy, dz, d2, t[1], t[2], t[3]);
-            t[0] = fadd(fadd(li, lj), scorr<N>(c.sc, d2));
-        },
-        [&](const float (&u)[4]) {
-            ax = ffma(u[0], u[1], ax);
-            ay = ffma(u[0], u[2], ay);
-            az = ffma(u[0], u[3], az);
-        });
-    dpx = fmul(gs, ax);
-    dpy = fmul(gs, ay);
-    dpz = fmul(gs, az);
-}
-
-// The thread's particle and lane in a launch of L lanes per particle; false
-// for threads past the last particle (whole groups) and, group-wide, once a
-// fatal status bit is set.
-template <int L>
-__device__ __forceinline__ bool group_thread(int n, const unsigned* status, int& i, int& sub,
-                                             unsigned& gmask) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    i = t / L;
-    sub = t % L;
-    gmask = 0u;
-    if (i >= n) return false;
-    if constexpr (L == 1) {
-        return !fatal(status);
-    } else {
-        gmask = lane_group_mask<L>();
-        return !__any_sync(gmask, fatal(status));
-    }
-}
-
 // delta p + applyDeltaPosition + CollisionSystem::solve + next cell keys.
 // N: artificial-pressure exponent fixed at compile time (0 = read at run time).
-// moved (optional): bit a set where the projection changed component a.
-// pre (optional): the position before the projection.
-// L lanes per particle share the neighbour terms (small scenes, with the
-// split walks); lane 0 applies.
-template <int N, bool B, int L>
+// moved, pre: see apply_delta.
+template <int N, bool B>
 __global__ void PBF_GATHER_REGS(48)
 k_delta_apply(const float4* __restrict__ xs, const uint32_t* __restrict__ nbr,
               const int* __restrict__ cnt, const float* __restrict__ lam, StepConst c, int n,
               float4* __restrict__ xs_out, uint32_t* __restrict__ keys_out, CellBins bins,
               uint8_t* __restrict__ moved, float4* __restrict__ pre,
               unsigned* __restrict__ status) {
-    int i, sub;
-    unsigned gmask;
-    if (!group_thread<L>(n, status, i, sub, gmask)) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n || fatal(status)) return;
     const float4 pi = xs[i];
     const int count = cnt[i];
     float dpx, dpy, dpz;
@@ -977,27 +589,9 @@ k_delta_apply(const float4* __restrict__ xs, const uint32_t* __restrict__ nbr,
         dpx = dpy = dpz = CUDART_NAN_F;
     } else {
         const float gs = B ? scene_of(c, i).gs : c.gs;
-        if constexpr (L == 1)
-            delta_sum<N>(c, xs, nbr, lam, i, count, pi, gs, dpx, dpy, dpz);
-        else
-            delta_sum_group<N, L>(c, xs, nbr, lam, i, sub, gmask, count, pi, gs, dpx, dpy, dpz);
+        delta_sum<N>(c, xs, nbr, lam, i, count, pi, gs, dpx, dpy, dpz);
     }
-    if (sub != 0) return;
-    float px = fadd(pi.x, dpx), py = fadd(pi.y, dpy), pz = fadd(pi.z, dpz);
-    const float ux = px, uy = py, uz = pz;
-    if (pre) pre[i] = make_float4(ux, uy, uz, pi.w);
-    if (!project_all(colliders_of<B>(c, i), c.particle_radius, px, py, pz))
-        atomicOr(status, kStatusNotConverged);
-    if (moved)
-        moved[i] = static_cast<uint8_t>((px != ux) | ((py != uy) << 1) | ((pz != uz) << 2));
-    const float4 q = make_float4(px, py, pz, pi.w);
-    xs_out[i] = q;
-    if (keys_out) {
-        GridConst g;
-        uint32_t base;
-        grid_of<B>(c, i, g, base);
-        put_key(keys_out, bins, i, base + key_of(g, q));
-    }
+    apply_delta<B>(c, i, pi, dpx, dpy, dpz, xs_out, keys_out, bins, moved, pre, status);
 }
 
 // Gather x, v_in, v.w and ids through the composite permutation of the
@@ -1111,62 +705,6 @@ k_search_xsph(const float4* __restrict__ xs, const float* __restrict__ sx,
     xsph_tail<B>(c, i, pi, xs, nbr, count, cnt, v, v_out, vin, resolve, status);
 }
 
-// k_search_xsph with L lanes per particle: the group walks together
-// (walk_chunks) and shares the XSPH terms; lane 0 writes.
-template <bool B, int L>
-__global__ void __launch_bounds__(kMaxTunedBlock)
-k_search_xsph_split(const float4* __restrict__ xs, const float* __restrict__ sx,
-                    const float* __restrict__ sy, const float* __restrict__ sz,
-                    const int* __restrict__ first, StepConst c, int n,
-                    uint32_t* __restrict__ nbr, int* __restrict__ cnt,
-                    const float4* __restrict__ v, float4* __restrict__ v_out,
-                    const float4* __restrict__ vin, bool resolve, unsigned* __restrict__ status) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = t / L, sub = t % L;
-    if (i >= n) return;  // whole groups
-    const unsigned gmask = lane_group_mask<L>();
-    if (__any_sync(gmask, fatal(status))) return;
-    const float4 pi = xs[i];
-    const int count =
-        walk_chunks<B, L>(c, i, sub, gmask, pi, sx, sy, sz, first, nbr + nb_first(c, i));
-    if (sub == 0) {
-        cnt[i] = count;
-        if (count > c.max_nb) atomicOr(status, kStatusNeighborOverflow);
-    }
-    // applyXsphViscosity over the new list, its terms spread over the group.
-    const float4 vi = v[i];
-    float4 out;
-    if (!count_ok(count, c.max_nb)) {
-        out = make_float4(CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F, vi.w);
-    } else {
-        const uint32_t* row = nbr + nb_first(c, i);
-        const size_t st = nb_step(c);
-        float cx = 0.0f, cy = 0.0f, cz = 0.0f;
-        group_sum<L, 4>(
-            count, sub, gmask,
-            [&](int k, float (&t)[4]) {
-                const uint32_t j = row[static_cast<size_t>(k) * st];  // written above
-                const float4 pj = __ldg(&xs[j]), vj = __ldg(&v[j]);
-                t[0] = poly6(c.k, dist2(fsub(pi.x, pj.x), fsub(pi.y, pj.y), fsub(pi.z, pj.z)));
-                t[1] = fsub(vj.x, vi.x);
-                t[2] = fsub(vj.y, vi.y);
-                t[3] = fsub(vj.z, vi.z);
-            },
-            [&](const float (&u)[4]) {
-                cx = ffma(u[1], u[0], cx);
-                cy = ffma(u[2], u[0], cy);
-                cz = ffma(u[3], u[0], cz);
-            });
-        const float xc = B ? scene_of(c, i).xsph_c : c.xsph_c;
-        out = make_float4(ffma(xc, cx, vi.x), ffma(xc, cy, vi.y), ffma(xc, cz, vi.z), vi.w);
-    }
-    if (sub != 0) return;
-    if (resolve)
-        resolve_velocity(colliders_of<B>(c, i), c.particle_radius, c.restitution, c.friction, pi,
-                         vin[i], out);
-    v_out[i] = out;
-}
-
 // computeVorticity (pbf_solver_kernels.cu:268-315).
 __global__ void __launch_bounds__(kMaxTunedBlock)
 k_vorticity(const float4* __restrict__ x, const float4* __restrict__ v,
@@ -1223,22 +761,6 @@ __global__ void __launch_bounds__(kBlock) k_omega_norm(float4* __restrict__ om, 
     om[i] = w;
 }
 
-// The confinement velocity from the summed eta = sum (|w_j| - |w_i|) grad W.
-__device__ __forceinline__ float4 confine_finish(const StepConst& c, float ex, float ey, float ez,
-                                                 float4 wi, float4 vi) {
-    const float el = len3(ex, ey, ez);
-    float nx = 0.0f, ny = 0.0f, nz = 0.0f;
-    if (el > kEtaEpsilon) {
-        nx = fdiv(ex, el);
-        ny = fdiv(ey, el);
-        nz = fdiv(ez, el);
-    }
-    const float cx = fmul(c.vort_eps, crossc(ny, nz, wi.y, wi.z));
-    const float cy = fmul(c.vort_eps, crossc(nz, nx, wi.z, wi.x));
-    const float cz = fmul(c.vort_eps, crossc(nx, ny, wi.x, wi.y));
-    return make_float4(ffma(c.dt, cx, vi.x), ffma(c.dt, cy, vi.y), ffma(c.dt, cz, vi.z), vi.w);
-}
-
 // applyVorticityConfinement (pbf_solver_kernels.cu:317-385).
 __device__ __forceinline__ float4 confine_one(const StepConst& c, const float4* __restrict__ x,
                                               const uint32_t* __restrict__ nbr, int count,
@@ -1292,49 +814,6 @@ k_confine(const float4* __restrict__ x, const uint32_t* __restrict__ nbr,
         resolve_velocity(colliders_of<B>(c, i), c.particle_radius, c.restitution, c.friction,
                          x[i], vin[i], out);
     v_out[i] = out;
-}
-
-// k_vorticity with L lanes per particle sharing the neighbour terms (small
-// scenes); lane 0 writes.
-template <int L>
-__global__ void __launch_bounds__(kMaxTunedBlock)
-k_vorticity_group(const float4* __restrict__ x, const float4* __restrict__ v,
-                  const uint32_t* __restrict__ nbr, const int* __restrict__ cnt, StepConst c,
-                  int n, float4* __restrict__ omega, bool store_norm,
-                  const unsigned* __restrict__ status) {
-    int i, sub;
-    unsigned gmask;
-    if (!group_thread<L>(n, status, i, sub, gmask)) return;
-    const int count = cnt[i];
-    if (!count_ok(count, c.max_nb)) {
-        if (sub == 0)
-            omega[i] = make_float4(CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F,
-                                   store_norm ? CUDART_NAN_F : 0.0f);
-        return;
-    }
-    const float4 pi = x[i], vi = v[i];
-    const uint32_t* row = nbr + nb_first(c, i);
-    const size_t st = nb_step(c);
-    float ox = 0.0f, oy = 0.0f, oz = 0.0f;
-    group_sum<L, 3>(
-        count, sub, gmask,
-        [&](int k, float (&t)[3]) {
-            const uint32_t j = __ldg(&row[static_cast<size_t>(k) * st]);
-            const float4 pj = __ldg(&x[j]), vj = __ldg(&v[j]);
-            const float dx = fsub(pi.x, pj.x), dy = fsub(pi.y, pj.y), dz = fsub(pi.z, pj.z);
-            float gx, gy, gz;
-            spiky(c.k, dx, dy, dz, dist2(dx, dy, dz), gx, gy, gz);
-            const float vx = fsub(vj.x, vi.x), vy = fsub(vj.y, vi.y), vz = fsub(vj.z, vi.z);
-            t[0] = crossc(gy, gz, vy, vz);
-            t[1] = crossc(gz, gx, vz, vx);
-            t[2] = crossc(gx, gy, vx, vy);
-        },
-        [&](const float (&u)[3]) {
-            ox = fadd(ox, u[0]);
-            oy = fadd(oy, u[1]);
-            oz = fadd(oz, u[2]);
-        });
-    if (sub == 0) omega[i] = make_float4(ox, oy, oz, store_norm ? len3(ox, oy, oz) : 0.0f);
 }
 
 template <bool B>
@@ -1484,66 +963,42 @@ void launch_gather_first(const uint32_t* perm, const float4* xs_in, float4* xs_o
     launch_k(k_gather_first, blocks_for(threads), kBlock, st, perm, xs_in, xs_out, org_in, org_out,
              sx, sy, sz, n, skeys, static_cast<uint32_t>(cells), first, status);
 }
-inline int tuned_block(const StepConst& c, int k) { return c.blk[k] > 0 ? c.blk[k] : kBlock; }
+inline int tuned_block(const StepConst& c, int k) {
+    return c.blk[k] > 0 ? c.blk[k] : (c.walk_lanes > 1 ? kGroupBlock : kBlock);
+}
 
-// Scene sizes for which a group of 8 or 4 lanes walks each particle by
-// default.  Measured steps of dam breaks at 1 / 4 / 8 lanes: 0.219 / 0.206 /
-// 0.174 ms at 8,192 particles, 0.270 / 0.230 / 0.215 at 16,384, 0.249 / 0.242
-// / 0.237 at 20,480, 0.262 / 0.247 / 0.268 at 24,576, 0.269 / 0.255 / 0.291 at
-// 28,672 and 0.274 / 0.283 / 0.334 at 32,768; 2 lanes are slower than 1 or 4
-// (0.329 ms at 16,384, 0.399 at 65,536 against 0.316 for 1 lane: from there
-// on the GPU is full with one lane per particle).
-constexpr size_t kSplitWalk8Max = 20480;
-constexpr size_t kSplitWalk4Below = size_t(1) << 15;
+// Lanes per particle of the neighbour kernels by default (the walks take nine,
+// a stencil row each, from 2 on).  Fewer lanes do less work in all, more make
+// a shorter launch.  Measured steps of dam breaks in motion at 1 / 8 / 16 / 32
+// lanes: 162 / 98 / 92 / 88 us at 1,024 particles, 190 / 108 / 103 / 99 at
+// 2,048, 197 / 115 / 109 / 109 at 4,096, 206 / 131 / 128 / 144 at 8,192, 222 /
+// 165 / 173 / 193 at 13,824, 228 / 178 / 192 / 214 at 16,384, 231 / 235 / 252 /
+// 287 at 24,576 and 236 / 281 / 296 / 340 at 32,768 (three lanes with a plane
+// of rows each for the walk: 225 at 24,576, 250 at 32,768).
+constexpr size_t kLanes32Max = 3072, kLanes16Max = 10240, kLanes8Max = 22528;
 
-// Lanes per particle of a launch: c.walk_lanes where the split walk applies.
-inline int split_lanes(const StepConst& c, int n) {
+// Lanes per particle of a launch: c.walk_lanes where the group kernels apply.
+inline int group_lanes(const StepConst& c, int n) {
     const int L = c.walk_lanes;
-    if ((L != 2 && L != 4 && L != 8) || c.nb_off != nullptr || c.max_nb < L ||
-        static_cast<long long>(n) * L > (1LL << 30))
+    // The walks start 32 threads for three particles.
+    if (L < 2 || c.nb_off != nullptr || c.max_nb < L ||
+        static_cast<long long>(n) * std::max(L, 11) > (1LL << 30))
         return 1;
     return L;
 }
 
 int default_walk_lanes(size_t n, int max_nb) {
-    int L = n <= kSplitWalk8Max ? 8 : (n < kSplitWalk4Below ? 4 : 1);
+    int L = n <= kLanes32Max ? 32 : (n <= kLanes16Max ? 16 : (n <= kLanes8Max ? 8 : 1));
     while (L > 1 && max_nb < L) L /= 2;  // a group never has more lanes than list slots
     return L;
-}
-
-template <bool LAMBDA, bool B>
-void launch_search_split(int L, int bs, const float4* xs, const float* sx, const float* sy,
-                         const float* sz, const int* first, const StepConst& c, int n,
-                         uint32_t* nbr, int* cnt, float* lam, unsigned* status, cudaStream_t st) {
-    const unsigned g = blocks_for(static_cast<size_t>(n) * L, bs);
-    if (L == 8)
-        launch_k(k_search_split<LAMBDA, B, 8>, g, bs, st, xs, sx, sy, sz, first, c, n, nbr, cnt,
-                 lam, status);
-    else if (L == 4)
-        launch_k(k_search_split<LAMBDA, B, 4>, g, bs, st, xs, sx, sy, sz, first, c, n, nbr, cnt,
-                 lam, status);
-    else
-        launch_k(k_search_split<LAMBDA, B, 2>, g, bs, st, xs, sx, sy, sz, first, c, n, nbr, cnt,
-                 lam, status);
 }
 
 void launch_search(const float4* xs, const float* sx, const float* sy, const float* sz,
                    const int* first, const StepConst& c, int n, uint32_t* nbr, int* cnt, float* lam,
                    unsigned* status, bool with_lambda, cudaStream_t st) {
     const int bs = tuned_block(c, with_lambda ? kTunedSearchLambda : kTunedSearch);
-    if (const int L = split_lanes(c, n); L > 1) {
-        if (with_lambda && c.scenes)
-            launch_search_split<true, true>(L, bs, xs, sx, sy, sz, first, c, n, nbr, cnt, lam,
-                                            status, st);
-        else if (with_lambda)
-            launch_search_split<true, false>(L, bs, xs, sx, sy, sz, first, c, n, nbr, cnt, lam,
-                                             status, st);
-        else if (c.scenes)
-            launch_search_split<false, true>(L, bs, xs, sx, sy, sz, first, c, n, nbr, cnt, lam,
-                                             status, st);
-        else
-            launch_search_split<false, false>(L, bs, xs, sx, sy, sz, first, c, n, nbr, cnt, lam,
-                                              status, st);
+    if (group_lanes(c, n) > 1) {
+        launch_search_rows(bs, xs, sx, sy, sz, first, c, n, nbr, cnt, lam, status, with_lambda, st);
         return;
     }
     const unsigned g = blocks_for(n, bs);
@@ -1561,36 +1016,14 @@ void launch_search(const float4* xs, const float* sx, const float* sy, const flo
                  status);
 }
 
-template <bool B>
-void launch_search_xsph_split(int L, unsigned g, int bs, const float4* xs, const float* sx,
-                              const float* sy, const float* sz, const int* first,
-                              const StepConst& c, int n, uint32_t* nbr, int* cnt, const float4* v,
-                              float4* v_out, const float4* vin, bool resolve, unsigned* status,
-                              cudaStream_t st) {
-    if (L == 8)
-        launch_k(k_search_xsph_split<B, 8>, g, bs, st, xs, sx, sy, sz, first, c, n, nbr, cnt, v,
-                 v_out, vin, resolve, status);
-    else if (L == 4)
-        launch_k(k_search_xsph_split<B, 4>, g, bs, st, xs, sx, sy, sz, first, c, n, nbr, cnt, v,
-                 v_out, vin, resolve, status);
-    else
-        launch_k(k_search_xsph_split<B, 2>, g, bs, st, xs, sx, sy, sz, first, c, n, nbr, cnt, v,
-                 v_out, vin, resolve, status);
-}
-
 void launch_search_xsph(const float4* xs, const float* sx, const float* sy, const float* sz,
                         const int* first, const StepConst& c, int n, uint32_t* nbr, int* cnt,
                         const float4* v, float4* v_out, const float4* vin, bool resolve,
                         unsigned* status, cudaStream_t st) {
     const int bs = tuned_block(c, kTunedSearch);
-    if (const int L = split_lanes(c, n); L > 1) {
-        const unsigned g = blocks_for(static_cast<size_t>(n) * L, bs);
-        if (c.scenes)
-            launch_search_xsph_split<true>(L, g, bs, xs, sx, sy, sz, first, c, n, nbr, cnt, v,
-                                           v_out, vin, resolve, status, st);
-        else
-            launch_search_xsph_split<false>(L, g, bs, xs, sx, sy, sz, first, c, n, nbr, cnt, v,
-                                            v_out, vin, resolve, status, st);
+    if (group_lanes(c, n) > 1) {
+        launch_search_xsph_rows(bs, xs, sx, sy, sz, first, c, n, nbr, cnt, v, v_out, vin, resolve,
+                                status, st);
         return;
     }
     const unsigned g = blocks_for(n, bs);
@@ -1635,30 +1068,22 @@ void launch_delta_apply_b(const float4* xs, const uint32_t* nbr, const int* cnt,
                           const CellBins& bins, uint8_t* moved, float4* pre, unsigned* status,
                           cudaStream_t st) {
     const int bs = tuned_block(c, kTunedDelta);
-    const unsigned g = blocks_for(n, bs);
-    const int L = split_lanes(c, n);
-    const unsigned gl = blocks_for(static_cast<size_t>(n) * L, bs);
-#define PBF_DELTA_CASE(N)                                                                        \
-    if (L == 8)                                                                                  \
-        launch_k(k_delta_apply<N, B, 8>, gl, bs, st, xs, nbr, cnt, lam, c, n, xs_out, keys_out,  \
-                 bins, moved, pre, status);                                                            \
-    else if (L == 4)                                                                             \
-        launch_k(k_delta_apply<N, B, 4>, gl, bs, st, xs, nbr, cnt, lam, c, n, xs_out, keys_out,  \
-                 bins, moved, pre, status);                                                            \
-    else if (L == 2)                                                                             \
-        launch_k(k_delta_apply<N, B, 2>, gl, bs, st, xs, nbr, cnt, lam, c, n, xs_out, keys_out,  \
-                 bins, moved, pre, status);                                                            \
-    else                                                                                         \
-        launch_k(k_delta_apply<N, B, 1>, g, bs, st, xs, nbr, cnt, lam, c, n, xs_out, keys_out,   \
-                 bins, moved, pre, status)
-    switch (c.sc.k != 0.0f ? c.sc.n : 0) {
-        case 1: PBF_DELTA_CASE(1); break;
-        case 2: PBF_DELTA_CASE(2); break;
-        case 3: PBF_DELTA_CASE(3); break;
-        case 4: PBF_DELTA_CASE(4); break;
-        default: PBF_DELTA_CASE(0); break;
+    if (const int L = group_lanes(c, n); L > 1) {
+        launch_delta_group(L, bs, xs, nbr, cnt, lam, c, n, xs_out, keys_out, bins, moved, pre,
+                           status, st);
+        return;
     }
-#undef PBF_DELTA_CASE
+    auto run = [&](auto k) {
+        launch_k(k, blocks_for(n, bs), bs, st, xs, nbr, cnt, lam, c, n, xs_out, keys_out, bins,
+                 moved, pre, status);
+    };
+    switch (c.sc.k != 0.0f ? c.sc.n : 0) {
+        case 1: run(k_delta_apply<1, B>); break;
+        case 2: run(k_delta_apply<2, B>); break;
+        case 3: run(k_delta_apply<3, B>); break;
+        case 4: run(k_delta_apply<4, B>); break;
+        default: run(k_delta_apply<0, B>); break;
+    }
 }
 void launch_delta_apply(const float4* xs, const uint32_t* nbr, const int* cnt, const float* lam,
                         const StepConst& c, int n, float4* xs_out, uint32_t* keys_out,
@@ -1693,20 +1118,12 @@ void launch_vorticity(const float4* x, const float4* v, const uint32_t* nbr, con
                       const StepConst& c, int n, float4* omega, bool store_norm,
                       const unsigned* status, cudaStream_t st) {
     const int bs = tuned_block(c, kTunedVorticity);
-    const int L = split_lanes(c, n);
-    const unsigned gl = blocks_for(static_cast<size_t>(n) * L, bs);
-    if (L == 8)
-        launch_k(k_vorticity_group<8>, gl, bs, st, x, v, nbr, cnt, c, n, omega, store_norm,
-                 status);
-    else if (L == 4)
-        launch_k(k_vorticity_group<4>, gl, bs, st, x, v, nbr, cnt, c, n, omega, store_norm,
-                 status);
-    else if (L == 2)
-        launch_k(k_vorticity_group<2>, gl, bs, st, x, v, nbr, cnt, c, n, omega, store_norm,
-                 status);
-    else
-        launch_k(k_vorticity, blocks_for(n, bs), bs, st, x, v, nbr, cnt, c, n, omega, store_norm,
-                 status);
+    if (const int L = group_lanes(c, n); L > 1) {
+        launch_vorticity_group(L, bs, x, v, nbr, cnt, c, n, omega, store_norm, status, st);
+        return;
+    }
+    launch_k(k_vorticity, blocks_for(n, bs), bs, st, x, v, nbr, cnt, c, n, omega, store_norm,
+             status);
 }
 void launch_omega_norm(float4* omega, int n, cudaStream_t st) {
     launch_k(k_omega_norm, blocks_for(n), kBlock, st, omega, n);
@@ -1715,6 +1132,10 @@ void launch_confine(const float4* x, const uint32_t* nbr, const int* cnt, const 
                     const float4* v, const StepConst& c, int n, float4* v_out,
                     const float4* vin, bool resolve, const unsigned* status, cudaStream_t st) {
     const int bs = tuned_block(c, kTunedConfine);
+    if (const int L = group_lanes(c, n); L > 1) {
+        launch_confine_group(L, bs, x, nbr, cnt, omega, v, c, n, v_out, vin, resolve, status, st);
+        return;
+    }
     if (c.scenes)
         launch_k(k_confine<true>, blocks_for(n, bs), bs, st, x, nbr, cnt, omega, v, c, n, v_out,
                  vin, resolve, status);

@@ -43,9 +43,10 @@ struct StepConst {
     // nb_cap entries.  Null: slot-major lists, nbr[k * stride + i].
     const uint32_t* nb_off;
     size_t nb_cap;
-    // Lanes per particle in the list-writing walks (1, 2 or 4; 0 = 1): more
-    // than one splits each particle's stencil rows over a lane group, for
-    // scenes too small to fill the GPU.  Slot-major lists only.
+    // Lanes per particle in the neighbour kernels (1, 2, 4, 8, 16 or 32; 0 =
+    // 1): more than one shares each particle's work over a lane group
+    // (pbf_group.cu), for scenes too small to fill the GPU.  Slot-major lists
+    // only.
     int walk_lanes;
     // Leave out of the walks the stencil cells that cannot hold a neighbour
     // (their box is farther than h from the particle).  Needs cell tables
@@ -54,8 +55,8 @@ struct StepConst {
     bool prune_cells;
 };
 
-// Lanes per particle for the walks of an n-particle scene (slot-major lists
-// with max_nb slots).
+// Lanes per particle for the neighbour kernels of an n-particle scene
+// (slot-major lists with max_nb slots).
 int default_walk_lanes(size_t n, int max_nb);
 
 // Stride (floats) of the x, y, z component arrays the walks read, for n
@@ -72,24 +73,35 @@ enum TunedKernel { kTunedSearchLambda, kTunedDelta, kTunedSearch, kTunedXsph, kT
 constexpr int kMaxTunedBlock = 512;
 
 constexpr int kBlock = 256;
+constexpr int kGroupBlock = 128;  // the neighbour kernels of small scenes
 
 inline unsigned blocks_for(size_t n, int block = kBlock) {
     return static_cast<unsigned>((n + block - 1) / block);
 }
 
-// Launches kernel k on stream st; launch errors throw like cuda_check.
+// Launches kernel k on stream st (launch_k_smem: with smem bytes of dynamic
+// shared memory per block); launch errors throw like cuda_check.
 void launch_error_check(cudaError_t e);
 template <typename... P, typename... A>
-inline void launch_k(void (*k)(P...), unsigned grid, unsigned block, cudaStream_t st, A&&... a) {
+inline void launch_k_smem(void (*k)(P...), unsigned grid, unsigned block, size_t smem,
+                          cudaStream_t st, A&&... a) {
     if (grid == 0) return;
+    if (smem > 48 * 1024)  // above the default limit a kernel has to opt in
+        launch_error_check(cudaFuncSetAttribute(reinterpret_cast<const void*>(k),
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                static_cast<int>(smem)));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = nullptr;
     cfg.numAttrs = 0;
     launch_error_check(cudaLaunchKernelEx(&cfg, k, static_cast<P>(a)...));
+}
+template <typename... P, typename... A>
+inline void launch_k(void (*k)(P...), unsigned grid, unsigned block, cudaStream_t st, A&&... a) {
+    launch_k_smem(k, grid, block, 0, st, static_cast<A&&>(a)...);
 }
 
 // Counting-sort state of one solver (pbf_bins.cu): count[cell] (zero between
@@ -102,7 +114,8 @@ struct CellBins {
 
 // --- step kernels (pbf_kernels.cu) -----------------------------------------
 void launch_predict(const float4* x, const float4* v, float4* xs, float4* vin, uint32_t* keys,
-                    const CellBins& bins, int n, const StepConst& c, const unsigned* status, cudaStream_t st);
+                    const CellBins& bins, int n, const StepConst& c, const unsigned* status,
+                    cudaStream_t st);
 void launch_cell_ranges(const uint32_t* skeys, int* cell_start, int* cell_end, int n,
                         const unsigned* status, cudaStream_t st);
 // Reorders predicted positions (float4 and x/y/z component arrays for the
@@ -143,6 +156,28 @@ void launch_count(const float4* xs, const float* sx, const float* sy, const floa
 size_t nb_scan_scratch_words(size_t n);
 void launch_nb_scan(const int* cnt, uint32_t* off, size_t cap, int n, uint32_t* scratch,
                     unsigned* status, cudaStream_t st);
+// The neighbour kernels of small scenes (pbf_group.cu), bs threads per block:
+// the walks with a lane per stencil row, the others with L lanes per
+// particle.  The launchers here choose them by StepConst::walk_lanes.
+void launch_search_rows(int bs, const float4* xs, const float* sx, const float* sy,
+                        const float* sz, const int* first, const StepConst& c, int n,
+                        uint32_t* nbr, int* cnt, float* lam, unsigned* status, bool with_lambda,
+                        cudaStream_t st);
+void launch_search_xsph_rows(int bs, const float4* xs, const float* sx, const float* sy,
+                             const float* sz, const int* first, const StepConst& c, int n,
+                             uint32_t* nbr, int* cnt, const float4* v, float4* v_out,
+                             const float4* vin, bool resolve, unsigned* status, cudaStream_t st);
+void launch_delta_group(int L, int bs, const float4* xs, const uint32_t* nbr, const int* cnt,
+                        const float* lam, const StepConst& c, int n, float4* xs_out,
+                        uint32_t* keys_out, const CellBins& bins, uint8_t* moved, float4* pre,
+                        unsigned* status, cudaStream_t st);
+void launch_vorticity_group(int L, int bs, const float4* x, const float4* v, const uint32_t* nbr,
+                            const int* cnt, const StepConst& c, int n, float4* omega,
+                            bool store_norm, const unsigned* status, cudaStream_t st);
+void launch_confine_group(int L, int bs, const float4* x, const uint32_t* nbr, const int* cnt,
+                          const float4* omega, const float4* v, const StepConst& c, int n,
+                          float4* v_out, const float4* vin, bool resolve, const unsigned* status,
+                          cudaStream_t st);
 // id_new may be null (ids not carried).
 void launch_finalize(const uint32_t* org, const float4* x_old, const float4* vin_old,
                      const float4* v_old, const uint32_t* id_old, const float4* xs, int n,

@@ -106,11 +106,11 @@ __host__ inline KernelConst make_kernel_const(float h) {
 
 // poly6FromDistanceSquared (include/pbf/sph_helpers.cuh:13-34).
 __device__ __forceinline__ float poly6(const KernelConst& k, float d2) {
-    if (d2 >= k.h2) return 0.0f;
     const float t = ffma(-d2, k.inv_h2, 1.0f);
     const float t2 = fmul(t, t);
     const float t3 = fmul(t2, t);
-    return fmul(k.c_poly6, t3);
+    const float w = fmul(k.c_poly6, t3);
+    return d2 >= k.h2 ? 0.0f : w;
 }
 
 // poly6 of two squared distances (lane-wise identical to poly6).
@@ -167,19 +167,16 @@ __device__ __forceinline__ float spiky_scale(const KernelConst& k, float d2) {
     const float t = ffma(-r, k.inv_h, 1.0f);
     return fmul(fmul(k.c_spiky, fmul(t, t)), rr);
 }
+// (Zero as a scale of 0: d * 0 may be -0, which leaves every sum unchanged.)
 __device__ __forceinline__ void spiky(const KernelConst& k, float dx, float dy, float dz,
                                       float d2, float& gx, float& gy, float& gz) {
-    if (d2 < kSpikyMinD2 || d2 >= k.h2) {
-        gx = gy = gz = 0.0f;
-        return;
-    }
-    const float s = spiky_scale(k, d2);
+    const float sc = spiky_scale(k, d2);
+    const float s = d2 < kSpikyMinD2 || d2 >= k.h2 ? 0.0f : sc;
     gx = fmul(dx, s);
     gy = fmul(dy, s);
     gz = fmul(dz, s);
 }
-// The scale s of two squared distances, 0 where spiky() returns zero
-// (d * 0 may then be -0, which leaves every sum it enters unchanged).
+// The scale s of two squared distances, 0 where spiky() returns zero.
 __device__ __forceinline__ f32x2 spiky_scale2(const KernelConst& k, f32x2 d2) {
     const f32x2 rr = rsqrt_nt2(d2);
     const f32x2 r = mul2(d2, rr);

@@ -1204,7 +1204,7 @@ pbf_status pbf_block_sizes(const pbf_solver* s, int* sizes, int count) {
         return PBF_ERR_INVALID_ARGUMENT;
     }
     for (int k = 0; k < count && k < kTunedCount; ++k)
-        sizes[k] = s->tuned[k] > 0 ? s->tuned[k] : kBlock;
+        sizes[k] = s->tuned[k] > 0 ? s->tuned[k] : (s->walk_lanes() > 1 ? kGroupBlock : kBlock);
     return PBF_OK;
 }
 
@@ -1232,7 +1232,7 @@ pbf_status pbf_walk_lanes(const pbf_solver* s, int* lanes) {
         pbf::set_global_error("solver handle and lanes must not be null");
         return PBF_ERR_INVALID_ARGUMENT;
     }
-    *lanes = s->walk_lanes();
+    *lanes = std::min(s->walk_lanes(), 8);
     return PBF_OK;
 }
 
