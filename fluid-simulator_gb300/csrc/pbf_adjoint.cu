@@ -68,7 +68,11 @@ __device__ __forceinline__ float3 operator-(float3 a, float3 b) {
 __device__ __forceinline__ float3 operator*(float s, float3 a) {
     return make_float3(s * a.x, s * a.y, s * a.z);
 }
-__device__ __forceinline__ float dot3(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+// The rounding of the two products' sums is spelled out here and in hess(), so
+// that it does not move with the code around them.
+__device__ __forceinline__ float dot3(float3 a, float3 b) {
+    return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+}
 __device__ __forceinline__ float3 cross3(float3 a, float3 b) {
     return make_float3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
 }
@@ -109,14 +113,25 @@ __device__ __forceinline__ PairTerms pair_terms(const StepConst& c, float3 r) {
         // with ratio^(3n - 1) = (ratio^3)^(n - 1) ratio^2.
         const float ratio = (c.sc.h2 - d2) * c.sc.inv_den;
         const float r2 = ratio * ratio;
-        const float pm1 = ipow(r2 * ratio, c.sc.n - 1);
+        const float r3 = r2 * ratio;
+        float pm1;  // r3^(n - 1), the common exponents without a loop
+        switch (c.sc.n) {
+            case 1: pm1 = 1.0f; break;
+            case 2: pm1 = r3; break;
+            case 3: pm1 = ipow_c<2>(r3); break;
+            case 4: pm1 = ipow_c<3>(r3); break;
+            default: pm1 = ipow(r3, c.sc.n - 1); break;
+        }
         t.s = c.sc.negk * pm1 * r2 * ratio;
         t.sp = 3.0f * c.sc.k * static_cast<float>(c.sc.n) * pm1 * r2 * c.sc.inv_den;
     }
     return t;
 }
 __device__ __forceinline__ float3 hess(const PairTerms& t, float3 r, float3 u) {
-    return t.f * u + (t.fpr * dot3(r, u)) * r;
+    const float k = __fmul_rn(t.fpr, dot3(r, u));
+    return make_float3(__fmaf_rn(t.f, u.x, __fmul_rn(k, r.x)),
+                       __fmaf_rn(t.f, u.y, __fmul_rn(k, r.y)),
+                       __fmaf_rn(t.f, u.z, __fmul_rn(k, r.z)));
 }
 
 // The gather passes give each particle L consecutive threads (L = 2 or 4):
@@ -133,6 +148,30 @@ __device__ __forceinline__ float lane_sum(float v) {
 template <int L>
 __device__ __forceinline__ float3 lane_sum(float3 v) {
     return make_float3(lane_sum<L>(v.x), lane_sum<L>(v.y), lane_sum<L>(v.z));
+}
+
+// A lane's entries of particle i's list in order: use(load(j)) for each.  The
+// passes are bound by the latency of index and gather (two dependent reads an
+// entry), so the next entry's data and the index after it are on their way
+// while an entry is used.
+template <int L, class Load, class Use>
+__device__ __forceinline__ void for_lane_entries(const uint32_t* __restrict__ nbr, size_t stride,
+                                                 int i, int lane, int count, Load load, Use use) {
+    if (lane >= count) return;
+    const uint32_t* __restrict__ row = nbr + i;
+    int k = lane;
+    auto d = load(__ldg(&row[static_cast<size_t>(k) * stride]));
+    uint32_t j = k + L < count ? __ldg(&row[static_cast<size_t>(k + L) * stride]) : 0u;
+    for (;;) {
+        const bool more = k + L < count;
+        auto dn = d;
+        if (more) dn = load(j);
+        if (k + 2 * L < count) j = __ldg(&row[static_cast<size_t>(k + 2 * L) * stride]);
+        use(d);
+        if (!more) break;
+        d = dn;
+        k += L;
+    }
 }
 
 // ---- adjoint -----------------------------------------------------------------
@@ -334,16 +373,21 @@ __global__ void k_xsph_adj(const float4* __restrict__ pF, const float4* __restri
     const float3 pi = f3(pF[ii]), vi = f3(v2[ii]), gi = f3(gv3[ii]);
     const int count = live ? min(cnt[i], c.max_nb) : 0;
     float3 sg = make_float3(0.0f, 0.0f, 0.0f), sv = sg, pos = sg;
-    for (int k = lane; k < count; k += L) {
-        const uint32_t j = __ldg(&nbr[static_cast<size_t>(k) * c.stride + i]);
-        const float3 r = pi - f3(__ldg(&pF[j]));
-        const PairTerms t = pair_terms(c, r);
-        const float3 dv = f3(__ldg(&v2[j])) - vi;
-        const float3 gj = f3(__ldg(&gv3[j]));
-        sg = sg + t.w * (gj - gi);
-        sv = sv + t.w * dv;
-        pos = pos + dot3(gi - gj, dv) * t.gw;
-    }
+    struct Entry {
+        float3 p, v, g;
+    };
+    for_lane_entries<L>(
+        nbr, c.stride, i, lane, count,
+        [&](uint32_t j) {
+            return Entry{f3(__ldg(&pF[j])), f3(__ldg(&v2[j])), f3(__ldg(&gv3[j]))};
+        },
+        [&](const Entry& q) {
+            const PairTerms t = pair_terms(c, pi - q.p);
+            const float3 dv = q.v - vi;
+            sg = sg + t.w * (q.g - gi);
+            sv = sv + t.w * dv;
+            pos = pos + dot3(gi - q.g, dv) * t.gw;
+        });
     sg = lane_sum<L>(sg);
     sv = lane_sum<L>(sv);
     pos = lane_sum<L>(pos);
@@ -380,20 +424,28 @@ __global__ void k_iter_adj_a(const float4* __restrict__ p, const float* __restri
     const int count = live ? min(cnt[i], c.max_nb) : 0;
     float wsum = 0.0f, s2 = 0.0f, glam = 0.0f;
     float3 G = make_float3(0.0f, 0.0f, 0.0f), X = G, dpos = G;
-    for (int k = lane; k < count; k += L) {
-        const uint32_t j = __ldg(&nbr[static_cast<size_t>(k) * c.stride + i]);
-        const float3 r = pi - f3(__ldg(&p[j]));
-        const PairTerms t = pair_terms(c, r);
-        const float3 u = gqi - f3(__ldg(&gq[j]));
-        const float coef = li + __ldg(&lam[j]) + t.s;
-        wsum += t.w;
-        s2 += dot3(t.g, t.g);
-        G = G + t.g;
-        X = X + coef * t.g;
-        const float ug = dot3(u, t.g);
-        glam += ug;
-        dpos = dpos + coef * hess(t, r, u) + (2.0f * t.sp * ug) * r;
-    }
+    struct Entry {
+        float3 p, g;
+        float l;
+    };
+    for_lane_entries<L>(
+        nbr, c.stride, i, lane, count,
+        [&](uint32_t j) {
+            return Entry{f3(__ldg(&p[j])), f3(__ldg(&gq[j])), __ldg(&lam[j])};
+        },
+        [&](const Entry& q) {
+            const float3 r = pi - q.p;
+            const PairTerms t = pair_terms(c, r);
+            const float3 u = gqi - q.g;
+            const float coef = li + q.l + t.s;
+            wsum += t.w;
+            s2 += dot3(t.g, t.g);
+            G = G + t.g;
+            X = X + coef * t.g;
+            const float ug = dot3(u, t.g);
+            glam += ug;
+            dpos = dpos + coef * hess(t, r, u) + (2.0f * t.sp * ug) * r;
+        });
     wsum = lane_sum<L>(wsum) + c.k.c_poly6;
     s2 = lane_sum<L>(s2);
     glam = lane_sum<L>(glam);
@@ -444,15 +496,21 @@ __global__ void k_iter_adj_b(const float4* __restrict__ p, const float4* __restr
     const float gDi = ai4.w, ai = aa[ii];
     const int count = live ? min(cnt[i], c.max_nb) : 0;
     float3 acc = make_float3(0.0f, 0.0f, 0.0f);
-    for (int k = lane; k < count; k += L) {
-        const uint32_t j = __ldg(&nbr[static_cast<size_t>(k) * c.stride + i]);
-        const float3 r = pi - f3(__ldg(&p[j]));
-        const PairTerms t = pair_terms(c, r);
-        const float4 aj4 = __ldg(&aux[j]);
-        const float gDj = aj4.w;
-        const float3 w = (gDi + gDj) * t.g + gDi * Gi - gDj * f3(aj4);
-        acc = acc + (ai + __ldg(&aa[j])) * t.gw + (2.0f * c.gs2) * hess(t, r, w);
-    }
+    struct Entry {
+        float3 p;
+        float4 x;
+        float a;
+    };
+    for_lane_entries<L>(
+        nbr, c.stride, i, lane, count,
+        [&](uint32_t j) { return Entry{f3(__ldg(&p[j])), __ldg(&aux[j]), __ldg(&aa[j])}; },
+        [&](const Entry& q) {
+            const float3 r = pi - q.p;
+            const PairTerms t = pair_terms(c, r);
+            const float gDj = q.x.w;
+            const float3 w = (gDi + gDj) * t.g + gDi * Gi - gDj * f3(q.x);
+            acc = acc + (ai + q.a) * t.gw + (2.0f * c.gs2) * hess(t, r, w);
+        });
     acc = lane_sum<L>(acc);
     if (!live || lane != 0) return;
     const float3 gp = f3(gpart[i]) + acc;
@@ -489,11 +547,14 @@ __global__ void k_conf_adj_a(const float4* __restrict__ pF, const float4* __rest
     const float mi = om[ii].w;
     const int count = live ? min(cnt[i], c.max_nb) : 0;
     float3 eta = make_float3(0.0f, 0.0f, 0.0f);
-    for (int k = lane; k < count; k += L) {
-        const uint32_t j = __ldg(&nbr[static_cast<size_t>(k) * c.stride + i]);
-        const PairTerms t = pair_terms(c, pi - f3(__ldg(&pF[j])));
-        eta = eta + (__ldg(&om[j]).w - mi) * t.g;
-    }
+    struct Entry {
+        float3 p;
+        float m;
+    };
+    for_lane_entries<L>(
+        nbr, c.stride, i, lane, count,
+        [&](uint32_t j) { return Entry{f3(__ldg(&pF[j])), __ldg(&om[j].w)}; },
+        [&](const Entry& q) { eta = eta + (q.m - mi) * pair_terms(c, pi - q.p).g; });
     eta = lane_sum<L>(eta);
     if (!live || lane != 0) return;
     const float3 w = f3(om[i]);
@@ -529,14 +590,22 @@ __global__ void k_conf_adj_b(const float4* __restrict__ pF, const float4* __rest
     const int count = live ? min(cnt[i], c.max_nb) : 0;
     float gm = 0.0f;
     float3 pos = make_float3(0.0f, 0.0f, 0.0f);
-    for (int k = lane; k < count; k += L) {
-        const uint32_t j = __ldg(&nbr[static_cast<size_t>(k) * c.stride + i]);
-        const float3 r = pi - f3(__ldg(&pF[j]));
-        const PairTerms t = pair_terms(c, r);
-        const float3 sg = gei + f3(__ldg(&geta[j]));
-        gm -= dot3(sg, t.g);
-        pos = pos + (__ldg(&om[j]).w - mi) * hess(t, r, sg);
-    }
+    struct Entry {
+        float3 p, g;
+        float m;
+    };
+    for_lane_entries<L>(
+        nbr, c.stride, i, lane, count,
+        [&](uint32_t j) {
+            return Entry{f3(__ldg(&pF[j])), f3(__ldg(&geta[j])), __ldg(&om[j].w)};
+        },
+        [&](const Entry& q) {
+            const float3 r = pi - q.p;
+            const PairTerms t = pair_terms(c, r);
+            const float3 sg = gei + q.g;
+            gm -= dot3(sg, t.g);
+            pos = pos + (q.m - mi) * hess(t, r, sg);
+        });
     gm = lane_sum<L>(gm);
     pos = lane_sum<L>(pos);
     if (!live || lane != 0) return;
@@ -563,14 +632,21 @@ __global__ void k_vort_adj(const float4* __restrict__ pF, const float4* __restri
     const float3 pi = f3(pF[ii]), vi = f3(v3[ii]), gwi = f3(gw[ii]);
     const int count = live ? min(cnt[i], c.max_nb) : 0;
     float3 acc = make_float3(0.0f, 0.0f, 0.0f), pos = acc;
-    for (int k = lane; k < count; k += L) {
-        const uint32_t j = __ldg(&nbr[static_cast<size_t>(k) * c.stride + i]);
-        const float3 r = pi - f3(__ldg(&pF[j]));
-        const PairTerms t = pair_terms(c, r);
-        const float3 sg = gwi + f3(__ldg(&gw[j]));
-        acc = acc + cross3(sg, t.g);
-        pos = pos + hess(t, r, cross3(f3(__ldg(&v3[j])) - vi, sg));
-    }
+    struct Entry {
+        float3 p, g, v;
+    };
+    for_lane_entries<L>(
+        nbr, c.stride, i, lane, count,
+        [&](uint32_t j) {
+            return Entry{f3(__ldg(&pF[j])), f3(__ldg(&gw[j])), f3(__ldg(&v3[j]))};
+        },
+        [&](const Entry& q) {
+            const float3 r = pi - q.p;
+            const PairTerms t = pair_terms(c, r);
+            const float3 sg = gwi + q.g;
+            acc = acc + cross3(sg, t.g);
+            pos = pos + hess(t, r, cross3(q.v - vi, sg));
+        });
     acc = lane_sum<L>(acc);
     pos = lane_sum<L>(pos);
     if (!live || lane != 0) return;
@@ -603,13 +679,35 @@ inline unsigned grid(int n) { return static_cast<unsigned>((n + kB - 1) / kB); }
 inline unsigned grid_lanes(int n, int L) {
     return static_cast<unsigned>((static_cast<size_t>(n) * L + kB - 1) / kB);
 }
-// Lanes per particle of the gather passes: four while fewer than 2^17
-// particles leave the SMs short of warps, two above.  Backward time over
-// the solver's forward, 60 steps, lanes 1 / 2 / 4: 1.97 / 1.64 / 1.62 at
-// 65,536 particles, 2.04 / 1.89 / 1.95 at 262,144, 2.20 / 2.19 / 2.39 at
-// 1,048,576.
+// Lanes per particle of the gather passes: four below 2^17 particles, two
+// above.  The lanes set the order of the partial sums, so another number
+// rounds the gradients differently (3e-7 relative in the parameter
+// derivatives); backward of 4 steps (us) at 2 / 4 / 8 / 16 lanes: 528 / 373 /
+// 300 / 303 at 4,080 particles, 518 / 436 / 460 / 587 at 16,384, 850 / 961 /
+// 1,123 / 1,650 at 65,536, 2,563 / 2,794 / 3,624 / 5,833 at 262,144.
 constexpr int kLanesBelow = 1 << 17;
 inline int lanes_for(int n) { return n < kLanesBelow ? kLanes : 2; }
+
+// Sums of the particles' partial parameter derivatives in a fixed order (a
+// strided sum per thread, then a tree), into pinned memory.
+constexpr int kSumThreads = 1024;
+__global__ void __launch_bounds__(kSumThreads)
+k_sum_parts(const double* __restrict__ a, const double* __restrict__ b, int n, double* out) {
+    __shared__ double part[32];
+    const double* __restrict__ v = blockIdx.x == 0 ? a : b;
+    double s = 0.0;
+    for (int i = threadIdx.x; i < n; i += kSumThreads) s += v[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        s = part[threadIdx.x];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (threadIdx.x == 0) out[blockIdx.x] = s;
+    }
+}
 
 }  // namespace adj
 }  // namespace pbf
@@ -650,6 +748,9 @@ struct pbf_adjoint {
     DeviceBuffer states;
     // Checkpoints (x, v) every `every` steps.
     DeviceBuffer ckpt;
+    bool have_forward = false;  // ckpt holds a forward's states
+    // Pinned words the device writes: the parameter derivatives.
+    double* h_sums = nullptr;
     // The tape holds the last segment of the latest forward (recorded by the
     // forward itself, so the backward need not recompute it).
     bool tape_last = false;
@@ -668,12 +769,18 @@ struct pbf_adjoint {
 
     ~pbf_adjoint() {
         clear_graphs();
+        if (h_sums) cudaFreeHost(h_sums);
         if (stream) cudaStreamDestroy(stream);
     }
 
     void clear_graphs() {
         for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
         graphs.clear();
+    }
+    void drop_forward() {
+        have_forward = false;
+        tape_last = false;
+        steps_done = 0;
     }
 
     // Tape of step slot t.  float4 arrays: P(t, k) positions of sort k in its
@@ -731,6 +838,7 @@ struct pbf_adjoint {
         const std::array<int, 3> d = grid_dims_checked(lo, hi, p.smoothingRadius);
         cuda_check(cudaSetDevice(device));
         if (!stream) cuda_check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+        if (!h_sums) cuda_check(cudaMallocHost(&h_sums, 2 * sizeof(double)));
         clear_graphs();
         n = count;
         max_nb = maxnb;
@@ -822,8 +930,7 @@ struct pbf_adjoint {
             cuda_check(cudaMemsetAsync(b->get(), 0, b->bytes(), stream));
         cuda_check(cudaStreamSynchronize(stream));
         ckpt = DeviceBuffer();
-        tape_last = false;
-        steps_done = 0;
+        drop_forward();
     }
 
     // CollisionSystem setters for the differentiated step (kind 0 spheres, 1
@@ -845,9 +952,7 @@ struct pbf_adjoint {
         d_col = std::move(d);
         apply_colliders();
         clear_graphs();  // the graphs hold the old constants
-        ckpt = DeviceBuffer();
-        tape_last = false;
-        steps_done = 0;
+        drop_forward();
     }
     void apply_colliders() {
         const float4* base = d_col.as<float4>();
@@ -867,15 +972,16 @@ struct pbf_adjoint {
         p.restDensity = rest_density;
         p.xsphViscosity = xsph;
         validate_params(p);
+        drop_forward();
+        // The graphs hold the constants; unchanged ones keep them (a rollout
+        // sets its physics every time).
+        if (rest_density == prm.restDensity && xsph == prm.xsphViscosity) return;
         prm = p;
         c.rho0 = rest_density;
         c.gs = prm.particleMass / rest_density;
         c.gs2 = c.gs * c.gs;
         c.xsph_c = xsph;
         clear_graphs();  // the graphs hold the old constants
-        ckpt = DeviceBuffer();
-        tape_last = false;
-        steps_done = 0;
     }
 
     // Sort of the current keys into permutation rel, gather of src (the
@@ -1049,9 +1155,10 @@ struct pbf_adjoint {
         cuda_check(cudaSetDevice(device));
         const size_t f4b = n * sizeof(float4);
         const int nck = steps / every + 1;
-        ckpt = DeviceBuffer(static_cast<size_t>(nck) * 2 * f4b);
-        steps_done = 0;
-        tape_last = false;
+        drop_forward();
+        if (ckpt.bytes() < static_cast<size_t>(nck) * 2 * f4b)
+            ckpt.allocate(static_cast<size_t>(nck) * 2 * f4b);
+        have_forward = true;
         clear_status();
         cuda_check(cudaMemcpyAsync(SX(0), x0, f4b, cudaMemcpyDefault, stream));
         cuda_check(cudaMemcpyAsync(SV(0), v0, f4b, cudaMemcpyDefault, stream));
@@ -1097,7 +1204,7 @@ struct pbf_adjoint {
 
     void backward(const pbf_float4* gx_out, const pbf_float4* gv_out, pbf_float4* gx0,
                   pbf_float4* gv0, double* grho0, double* gxsph) {
-        if (n == 0 || !ckpt.get()) fail(PBF_ERR_LOGIC, "backward needs a forward first");
+        if (n == 0 || !have_forward) fail(PBF_ERR_LOGIC, "backward needs a forward first");
         if (!gx_out || !gv_out || !gx0 || !gv0)
             fail(PBF_ERR_INVALID_ARGUMENT, "null gradient pointer");
         cuda_check(cudaSetDevice(device));
@@ -1124,19 +1231,12 @@ struct pbf_adjoint {
         }
         cuda_check(cudaMemcpyAsync(gx0, gx.get(), f4b, cudaMemcpyDefault, stream));
         cuda_check(cudaMemcpyAsync(gv0, gv.get(), f4b, cudaMemcpyDefault, stream));
-        std::vector<double> hr(n), hc(n);
-        cuda_check(cudaMemcpyAsync(hr.data(), acc_r.get(), n * sizeof(double),
-                                   cudaMemcpyDeviceToHost, stream));
-        cuda_check(cudaMemcpyAsync(hc.data(), acc_c.get(), n * sizeof(double),
-                                   cudaMemcpyDeviceToHost, stream));
+        launch_k(adj::k_sum_parts, 2u, adj::kSumThreads, stream, acc_r.as<double>(),
+                 acc_c.as<double>(), static_cast<int>(n), h_sums);
         check_status();
-        double sr = 0.0, sc = 0.0;
-        for (size_t i = 0; i < n; ++i) {
-            sr += hr[i];
-            sc += hc[i];
-        }
-        if (grho0) *grho0 = sr;
-        if (gxsph) *gxsph = sc;
+        const volatile double* sums = h_sums;
+        if (grho0) *grho0 = sums[0];
+        if (gxsph) *gxsph = sums[1];
     }
 };
 
