@@ -62,22 +62,23 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* warp_sums, 
     return (warp ? before : 0u) + incl - v;
 }
 
-constexpr int kItems = 8;  // cells per thread in the scans
+// Cells per thread in the scans: few where the launch is short and its blocks
+// should be many, 8 for large tables.
+constexpr int kFew = 2, kMany = 8;
 
-// kItems consecutive counts of the thread (0 past the last cell).  The count
-// array is padded to a multiple of kItems cells (bin_count_words).
+// ITEMS consecutive counts of the thread (0 past the last cell).  The count
+// array is padded to a multiple of kMany cells (bin_count_words).
+template <int ITEMS>
 __device__ __forceinline__ uint32_t load_counts(const uint32_t* __restrict__ count, uint32_t at,
-                                                uint32_t cells, uint32_t (&v)[kItems]) {
+                                                uint32_t cells, uint32_t (&v)[ITEMS]) {
     uint32_t sum = 0u;
 #pragma unroll
-    for (int q = 0; q < kItems; q += 4) {
-        const uint4 w = at + q < cells ? __ldcg(reinterpret_cast<const uint4*>(count + at + q))
-                                       : make_uint4(0u, 0u, 0u, 0u);
+    for (int q = 0; q < ITEMS; q += 2) {
+        const uint2 w = at + q < cells ? __ldcg(reinterpret_cast<const uint2*>(count + at + q))
+                                       : make_uint2(0u, 0u);
         v[q] = w.x;
         v[q + 1] = w.y;
-        v[q + 2] = w.z;
-        v[q + 3] = w.w;
-        sum += w.x + w.y + w.z + w.w;
+        sum += w.x + w.y;
     }
     return sum;
 }
@@ -85,6 +86,7 @@ __device__ __forceinline__ uint32_t load_counts(const uint32_t* __restrict__ cou
 // Up to kSmallCells cells: every block scans all counts into shared memory
 // (32 KB at most, from L2) and places its particles; block 0 writes first[].
 constexpr int kSmallThreads = 1024;
+constexpr int kItems = kMany;
 constexpr uint32_t kSmallCells = kSmallThreads * kItems;
 __global__ void __launch_bounds__(kSmallThreads)
 k_bin_small(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ place,
@@ -96,7 +98,7 @@ k_bin_small(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ plac
     const uint32_t key = i < n ? keys[i] : 0u, at = i < n ? place[i] : 0u;
     uint32_t v[kItems], total;
     const uint32_t c0 = threadIdx.x * kItems;
-    const uint32_t sum = load_counts(count, c0, cells, v);
+    const uint32_t sum = load_counts<kItems>(count, c0, cells, v);
     if (__syncthreads_or(fatal(status))) return;
     uint32_t run = block_scan<kSmallThreads>(sum, warp_sums, total);
 #pragma unroll
@@ -113,48 +115,56 @@ k_bin_small(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ plac
 }
 
 constexpr int kScanThreads = 512;
-constexpr uint32_t kScanTile = kScanThreads * kItems;
-// Up to this many cells the scan's blocks sum the counts before their own
-// tile themselves; above, the tiles' sums come from a launch of their own.
-constexpr uint32_t kDirectCells = 8 * kScanTile;
+// Up to kDirectCells the scan's blocks sum the counts before their own tile
+// themselves; above, the tiles' sums come from a launch of their own (in the
+// words after the counts; at 32,768 cells 3.8 + 5.9 us against 5.4).  Tiles of
+// kFew cells a thread up to kFewCells (32,768 cells: 8.4 -> 5.4 us).
+constexpr uint32_t kDirectCells = 32768;
+constexpr uint32_t kFewCells = 1u << 20;
 
+template <int ITEMS>
 __global__ void __launch_bounds__(kScanThreads)
 k_bin_sums(const uint32_t* __restrict__ count, uint32_t cells, uint32_t* __restrict__ sums,
            const unsigned* __restrict__ status) {
     __shared__ uint32_t warp_sums[kScanThreads / 32];
-    if (fatal(status)) return;
-    uint32_t v[kItems], total;
+    if (__syncthreads_or(fatal(status))) return;
+    uint32_t v[ITEMS], total;
     block_scan<kScanThreads>(
-        load_counts(count, blockIdx.x * kScanTile + threadIdx.x * kItems, cells, v), warp_sums,
-        total);
+        load_counts<ITEMS>(count, (blockIdx.x * kScanThreads + threadIdx.x) * ITEMS, cells, v),
+        warp_sums, total);
     if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
 // sums: the tiles' sums, or null (every block sums the counts before its tile).
+template <int ITEMS>
 __global__ void __launch_bounds__(kScanThreads)
 k_bin_scan(const uint32_t* __restrict__ count, uint32_t cells, const uint32_t* __restrict__ sums,
            int* __restrict__ first, const unsigned* __restrict__ status) {
     __shared__ uint32_t warp_sums[2][kScanThreads / 32];
-    if (__syncthreads_or(fatal(status))) return;
+    uint32_t v[ITEMS], base, total;
+    const uint32_t c0 = (blockIdx.x * kScanThreads + threadIdx.x) * ITEMS;
+    const uint32_t sum = load_counts<ITEMS>(count, c0, cells, v);
     uint32_t before = 0u;
     if (sums) {
         for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kScanThreads) before += sums[t];
     } else {
-        uint32_t v[kItems];
-        for (uint32_t t = 0; t < blockIdx.x; ++t)
-            before += load_counts(count, t * kScanTile + threadIdx.x * kItems, cells, v);
+        const uint4* c4 = reinterpret_cast<const uint4*>(count);
+        const uint32_t end = blockIdx.x * (kScanThreads * ITEMS / 4);
+#pragma unroll 8
+        for (uint32_t t = threadIdx.x; t < end; t += kScanThreads) {
+            const uint4 w = __ldcg(&c4[t]);
+            before += w.x + w.y + w.z + w.w;
+        }
     }
-    uint32_t v[kItems], base, total;
-    const uint32_t c0 = blockIdx.x * kScanTile + threadIdx.x * kItems;
-    const uint32_t sum = load_counts(count, c0, cells, v);
+    if (__syncthreads_or(fatal(status))) return;
     block_scan<kScanThreads>(before, warp_sums[0], base);
     uint32_t run = base + block_scan<kScanThreads>(sum, warp_sums[1], total);
 #pragma unroll
-    for (int q = 0; q < kItems; ++q) {
+    for (int q = 0; q < ITEMS; ++q) {
         if (c0 + q <= cells) first[c0 + q] = static_cast<int>(run);
         run += v[q];
     }
-    if (c0 + kItems == cells) first[cells] = static_cast<int>(run);
+    if (c0 + ITEMS == cells) first[cells] = static_cast<int>(run);
 }
 
 __global__ void __launch_bounds__(kBlock)
@@ -202,8 +212,8 @@ bool bins_apply(size_t n, uint64_t cells) {
 }
 
 size_t bin_count_words(uint64_t cells) {
-    return static_cast<size_t>((cells + kItems - 1) / kItems * kItems +
-                               (cells + kScanTile - 1) / kScanTile);
+    const uint64_t tile = kScanThreads * (cells <= kFewCells ? kFew : kMany);
+    return static_cast<size_t>((cells + kMany - 1) / kMany * kMany + (cells + tile - 1) / tile);
 }
 
 void launch_bin_order(const CellBins& b, const uint32_t* keys, int* first, uint32_t* list, int n,
@@ -214,13 +224,16 @@ void launch_bin_order(const CellBins& b, const uint32_t* keys, int* first, uint3
                  b.count, n, nc, first, list, status);
         return;
     }
-    const unsigned tiles = blocks_for(nc, kScanTile);
+    const bool few = nc <= kFewCells;
+    const unsigned tiles = blocks_for(nc, kScanThreads * (few ? kFew : kMany));
     uint32_t* sums = nullptr;
     if (nc > kDirectCells) {
-        sums = b.count + (nc + kItems - 1) / kItems * kItems;
-        launch_k(k_bin_sums, tiles, kScanThreads, st, b.count, nc, sums, status);
+        sums = b.count + (nc + kMany - 1) / kMany * kMany;
+        launch_k(few ? k_bin_sums<kFew> : k_bin_sums<kMany>, tiles, kScanThreads, st, b.count, nc,
+                 sums, status);
     }
-    launch_k(k_bin_scan, tiles, kScanThreads, st, b.count, nc, sums, first, status);
+    launch_k(few ? k_bin_scan<kFew> : k_bin_scan<kMany>, tiles, kScanThreads, st, b.count, nc,
+             sums, first, status);
     launch_k(k_bin_scatter, blocks_for(n), kBlock, st, keys, b.place, first, n, list, status);
 }
 

@@ -963,8 +963,28 @@ void launch_gather_first(const uint32_t* perm, const float4* xs_in, float4* xs_o
     launch_k(k_gather_first, blocks_for(threads), kBlock, st, perm, xs_in, xs_out, org_in, org_out,
              sx, sy, sz, n, skeys, static_cast<uint32_t>(cells), first, status);
 }
-inline int tuned_block(const StepConst& c, int k) {
-    return c.blk[k] > 0 ? c.blk[k] : (c.walk_lanes > 1 ? kGroupBlock : kBlock);
+// Lanes per particle of a launch: c.walk_lanes where the group kernels apply.
+inline int group_lanes(const StepConst& c, int n) {
+    const int L = c.walk_lanes;
+    // The walks start 32 threads for three particles.
+    if (L < 2 || c.nb_off != nullptr || c.max_nb < L ||
+        static_cast<long long>(n) * std::max(L, 11) > (1LL << 30))
+        return 1;
+    return L;
+}
+
+// Threads per block of the neighbour kernels by default.  Smaller blocks even
+// out the last wave once there are several blocks an SM: frame at 256 / 128 /
+// 64 threads 302 / 288 / 289 us at 65,536 particles, 414 / 388 / 382 at 131,072,
+// 708 / 687 / 685 at 262,144, 2,389 / 2,331 / 2,349 at 1,048,576; 242 / 248 /
+// 248 at 32,768, and 7.47 / 7.60 / 7.69 ms for 256 batched scenes.
+constexpr size_t kBlock128From = 57344;
+int default_block(size_t n, int lanes, bool batched) {
+    if (lanes > 1) return kGroupBlock;
+    return n >= kBlock128From && !batched ? 128 : kBlock;
+}
+inline int tuned_block(const StepConst& c, int n, int k) {
+    return c.blk[k] > 0 ? c.blk[k] : default_block(n, group_lanes(c, n), c.scenes != nullptr);
 }
 
 // Lanes per particle of the neighbour kernels by default (the walks take nine,
@@ -977,16 +997,6 @@ inline int tuned_block(const StepConst& c, int k) {
 // of rows each for the walk: 225 at 24,576, 250 at 32,768).
 constexpr size_t kLanes32Max = 3072, kLanes16Max = 10240, kLanes8Max = 22528;
 
-// Lanes per particle of a launch: c.walk_lanes where the group kernels apply.
-inline int group_lanes(const StepConst& c, int n) {
-    const int L = c.walk_lanes;
-    // The walks start 32 threads for three particles.
-    if (L < 2 || c.nb_off != nullptr || c.max_nb < L ||
-        static_cast<long long>(n) * std::max(L, 11) > (1LL << 30))
-        return 1;
-    return L;
-}
-
 int default_walk_lanes(size_t n, int max_nb) {
     int L = n <= kLanes32Max ? 32 : (n <= kLanes16Max ? 16 : (n <= kLanes8Max ? 8 : 1));
     while (L > 1 && max_nb < L) L /= 2;  // a group never has more lanes than list slots
@@ -996,7 +1006,7 @@ int default_walk_lanes(size_t n, int max_nb) {
 void launch_search(const float4* xs, const float* sx, const float* sy, const float* sz,
                    const int* first, const StepConst& c, int n, uint32_t* nbr, int* cnt, float* lam,
                    unsigned* status, bool with_lambda, cudaStream_t st) {
-    const int bs = tuned_block(c, with_lambda ? kTunedSearchLambda : kTunedSearch);
+    const int bs = tuned_block(c, n, with_lambda ? kTunedSearchLambda : kTunedSearch);
     if (group_lanes(c, n) > 1) {
         launch_search_rows(bs, xs, sx, sy, sz, first, c, n, nbr, cnt, lam, status, with_lambda, st);
         return;
@@ -1020,7 +1030,7 @@ void launch_search_xsph(const float4* xs, const float* sx, const float* sy, cons
                         const int* first, const StepConst& c, int n, uint32_t* nbr, int* cnt,
                         const float4* v, float4* v_out, const float4* vin, bool resolve,
                         unsigned* status, cudaStream_t st) {
-    const int bs = tuned_block(c, kTunedSearch);
+    const int bs = tuned_block(c, n, kTunedSearch);
     if (group_lanes(c, n) > 1) {
         launch_search_xsph_rows(bs, xs, sx, sy, sz, first, c, n, nbr, cnt, v, v_out, vin, resolve,
                                 status, st);
@@ -1038,7 +1048,7 @@ void launch_search_xsph(const float4* xs, const float* sx, const float* sy, cons
 void launch_count(const float4* xs, const float* sx, const float* sy, const float* sz,
                   const int* first, const StepConst& c, int n, int* cnt, unsigned* status,
                   cudaStream_t st) {
-    const int bs = tuned_block(c, kTunedSearch);
+    const int bs = tuned_block(c, n, kTunedSearch);
     const unsigned g = blocks_for(n, bs);
     if (c.scenes)
         launch_k(k_count<true>, g, bs, st, xs, sx, sy, sz, first, c, n, cnt, status);
@@ -1067,7 +1077,7 @@ void launch_delta_apply_b(const float4* xs, const uint32_t* nbr, const int* cnt,
                           const StepConst& c, int n, float4* xs_out, uint32_t* keys_out,
                           const CellBins& bins, uint8_t* moved, float4* pre, unsigned* status,
                           cudaStream_t st) {
-    const int bs = tuned_block(c, kTunedDelta);
+    const int bs = tuned_block(c, n, kTunedDelta);
     if (const int L = group_lanes(c, n); L > 1) {
         launch_delta_group(L, bs, xs, nbr, cnt, lam, c, n, xs_out, keys_out, bins, moved, pre,
                            status, st);
@@ -1106,7 +1116,7 @@ void launch_finalize(const uint32_t* org, const float4* x_old, const float4* vin
 void launch_xsph(const float4* x, const float4* v, const uint32_t* nbr, const int* cnt,
                  const StepConst& c, int n, float4* v_out, const float4* vin, bool resolve,
                  const unsigned* status, cudaStream_t st) {
-    const int bs = tuned_block(c, kTunedXsph);
+    const int bs = tuned_block(c, n, kTunedXsph);
     if (c.scenes)
         launch_k(k_xsph<true>, blocks_for(n, bs), bs, st, x, v, nbr, cnt, c, n, v_out, vin,
                  resolve, status);
@@ -1117,7 +1127,7 @@ void launch_xsph(const float4* x, const float4* v, const uint32_t* nbr, const in
 void launch_vorticity(const float4* x, const float4* v, const uint32_t* nbr, const int* cnt,
                       const StepConst& c, int n, float4* omega, bool store_norm,
                       const unsigned* status, cudaStream_t st) {
-    const int bs = tuned_block(c, kTunedVorticity);
+    const int bs = tuned_block(c, n, kTunedVorticity);
     if (const int L = group_lanes(c, n); L > 1) {
         launch_vorticity_group(L, bs, x, v, nbr, cnt, c, n, omega, store_norm, status, st);
         return;
@@ -1131,7 +1141,7 @@ void launch_omega_norm(float4* omega, int n, cudaStream_t st) {
 void launch_confine(const float4* x, const uint32_t* nbr, const int* cnt, const float4* omega,
                     const float4* v, const StepConst& c, int n, float4* v_out,
                     const float4* vin, bool resolve, const unsigned* status, cudaStream_t st) {
-    const int bs = tuned_block(c, kTunedConfine);
+    const int bs = tuned_block(c, n, kTunedConfine);
     if (const int L = group_lanes(c, n); L > 1) {
         launch_confine_group(L, bs, x, nbr, cnt, omega, v, c, n, v_out, vin, resolve, status, st);
         return;

@@ -37,7 +37,7 @@ struct StepConst {
     // (scenes occupy fixed contiguous slot ranges); null for one scene.
     const SceneConst* scenes;
     const uint16_t* sid;
-    // Threads per block of the tuned kernels (TunedKernel order); 0 = kBlock.
+    // Threads per block of the tuned kernels (TunedKernel order); 0 = default_block.
     int blk[6];
     // Compact neighbour lists: particle i's list is nbr[nb_off[i] + k] inside
     // nb_cap entries.  Null: slot-major lists, nbr[k * stride + i].
@@ -58,6 +58,8 @@ struct StepConst {
 // Lanes per particle for the neighbour kernels of an n-particle scene
 // (slot-major lists with max_nb slots).
 int default_walk_lanes(size_t n, int max_nb);
+// Threads per block of the neighbour kernels that no tuning has set.
+int default_block(size_t n, int lanes, bool batched);
 
 // Stride (floats) of the x, y, z component arrays the walks read, for n
 // particles: a multiple of 64 (every array 256-byte aligned, so the walk's

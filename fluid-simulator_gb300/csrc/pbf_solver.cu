@@ -197,7 +197,7 @@ struct pbf_solver {
     std::vector<size_t> scene_off;
     DeviceBuffer scene_tab, scene_id;
 
-    // Threads per block of the tuned kernels (0 = the default 256).
+    // Threads per block of the tuned kernels (0 = default_block).
     int tuned[kTunedCount] = {};
     int tuned_lanes = 0;  // lanes per particle of the walks set by pbf_set_walk_lanes; 0 = default
     int sort_tile = 0;    // keys per radix-sort tile chosen by the autotuner; 0 = by size
@@ -1245,7 +1245,8 @@ pbf_status pbf_block_sizes(const pbf_solver* s, int* sizes, int count) {
         return PBF_ERR_INVALID_ARGUMENT;
     }
     for (int k = 0; k < count && k < kTunedCount; ++k)
-        sizes[k] = s->tuned[k] > 0 ? s->tuned[k] : (s->walk_lanes() > 1 ? kGroupBlock : kBlock);
+        sizes[k] = s->tuned[k] > 0 ? s->tuned[k]
+                                   : default_block(s->n, s->walk_lanes(), s->nscenes > 0);
     return PBF_OK;
 }
 

@@ -2,7 +2,8 @@
 
 Up to 8,192 cells one launch scans the counts in every block; up to 32,768 a
 scan's blocks sum the counts before them; above, tile sums come from a launch
-of their own; with far more cells than particles the radix sort orders them.
+of their own, with larger tiles above 2^20; with far more cells than particles
+the radix sort orders them.
 Shuffled particles, some alone, some dozens to a cell, some outside the
 grid: after two frames the working order (stable within a cell), the counts
 and the state equal the FP32 oracle's bit for bit, also on a solver whose last
@@ -15,10 +16,10 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 # dims, particles: 1 cell; 8,191 to 8,193 cells; 32,768 and 32,769; whole
-# tiles of 4,096; more than 8 n + 65,536 cells.
+# tiles; more than 2^20 cells; more than 8 n + 65,536 cells.
 GRIDS = [((1, 1, 1), 1), ((1, 1, 1), 190), ((8191, 1, 1), 1025), ((32, 16, 16), 1024),
          ((2731, 3, 1), 2047), ((32, 32, 32), 3000), ((331, 11, 9), 1500), ((64, 36, 32), 5000),
-         ((73, 70, 3), 300), ((100, 100, 10), 700)]
+         ((73, 70, 3), 300), ((128, 128, 65), 125000), ((100, 100, 10), 700)]
 
 
 def _scene(dims, n):
