@@ -23,7 +23,7 @@ __device__ __forceinline__ size_t nb_first(const StepConst& c, int i) {
     return c.nb_off ? static_cast<size_t>(__ldg(&c.nb_off[i])) : static_cast<size_t>(i);
 }
 __device__ __forceinline__ size_t nb_step(const StepConst& c) {
-    return c.nb_off ? size_t(1) : c.stride;
+    return c.nb_off ? static_cast<size_t>(__ldg(c.nb_step)) : c.stride;
 }
 
 // Grid and first global cell key of slot i: the scene's (B) or c.g.

@@ -39,9 +39,11 @@ struct StepConst {
     const uint16_t* sid;
     // Threads per block of the tuned kernels (TunedKernel order); 0 = default_block.
     int blk[6];
-    // Compact neighbour lists: particle i's list is nbr[nb_off[i] + k] inside
-    // nb_cap entries.  Null: slot-major lists, nbr[k * stride + i].
+    // Compact neighbour lists: particle i's list is nbr[nb_off[i] + k *
+    // nb_step[0]] inside nb_cap entries.  Null: slot-major lists,
+    // nbr[k * stride + i].
     const uint32_t* nb_off;
+    const uint32_t* nb_step;
     size_t nb_cap;
     // Lanes per particle in the neighbour kernels (1, 2, 4, 8, 16 or 32; 0 =
     // 1): more than one shares each particle's work over a lane group
@@ -150,14 +152,15 @@ void launch_delta_apply(const float4* xs, const uint32_t* nbr, const int* cnt, c
                         uint8_t* moved = nullptr,
                         float4* pre = nullptr);
 // Compact lists: neighbour counts of the walk (no list written), then the
-// exclusive scan of the counts into off (n + 1 entries; a total above cap
-// sets kStatusListOverflow).  scratch: nb_scan_scratch_words(n) words.
+// exclusive scan of the counts into the lists' offsets off (n entries) and
+// the step between their entries (a total above cap sets
+// kStatusListOverflow).  scratch: nb_scan_scratch_words(n) words.
 void launch_count(const float4* xs, const float* sx, const float* sy, const float* sz,
                   const int* first, const StepConst& c, int n, int* cnt, unsigned* status,
                   cudaStream_t st);
 size_t nb_scan_scratch_words(size_t n);
-void launch_nb_scan(const int* cnt, uint32_t* off, size_t cap, int n, uint32_t* scratch,
-                    unsigned* status, cudaStream_t st);
+void launch_nb_scan(const int* cnt, uint32_t* off, uint32_t* step, size_t cap, int n,
+                    uint32_t* scratch, unsigned* status, cudaStream_t st);
 // The neighbour kernels of small scenes (pbf_group.cu), bs threads per block:
 // the walks with a lane per stencil row, the others with L lanes per
 // particle.  The launchers here choose them by StepConst::walk_lanes.

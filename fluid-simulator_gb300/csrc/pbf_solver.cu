@@ -203,9 +203,9 @@ struct pbf_solver {
     int sort_tile = 0;    // keys per radix-sort tile chosen by the autotuner; 0 = by size
 
     // Compact neighbour lists (list_cap > 0): every rebuild counts the
-    // neighbours, scans the counts into nb_off and writes each particle's
-    // list contiguously into list_cap entries in all.  0: slot-major lists of
-    // max_nb slots per particle.
+    // neighbours, scans the counts into nb_off (the last word: the step
+    // between entries) and writes the lists into list_cap entries in all.
+    // 0: slot-major lists of max_nb slots per particle.
     size_t list_cap = 0;
     DeviceBuffer nb_off, nb_scratch;
 
@@ -309,6 +309,7 @@ struct pbf_solver {
         for (int k = 0; k < kTunedCount; ++k) c.blk[k] = tuned[k];
         if (list_cap > 0) {
             c.nb_off = nb_off.as<uint32_t>();
+            c.nb_step = nb_off.as<uint32_t>() + cap;
             c.nb_cap = list_cap;
         }
         c.walk_lanes = walk_lanes();
@@ -423,7 +424,8 @@ struct pbf_solver {
                 launch_count(P(xs), soa.as<float>(), soa.as<float>() + soa_stride(),
                              soa.as<float>() + 2 * soa_stride(), cell_first.as<int>(), c, N,
                              cnt.as<int>(), sp, st);
-                launch_nb_scan(cnt.as<int>(), nb_off.as<uint32_t>(), list_cap, N,
+                launch_nb_scan(cnt.as<int>(), nb_off.as<uint32_t>(),
+                               nb_off.as<uint32_t>() + cap, list_cap, N,
                                nb_scratch.as<uint32_t>(), sp, st);
             };
             for (int it = 0; it < prm.solverIterations; ++it) {
