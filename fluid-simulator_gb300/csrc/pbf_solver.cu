@@ -332,10 +332,10 @@ struct pbf_solver {
         clear_graphs();
     }
 
-    // The counting sort's state when the rebuilds of n particles use it.
+    // The counting sort's state when the rebuilds use it.
     CellBins cell_bins() const {
         CellBins b;
-        if (bin_count.get() && bins_apply(n, cells)) {
+        if (bin_count.get()) {
             b.count = bin_count.as<uint32_t>();
             b.place = akeys.as<uint32_t>();
         }
@@ -752,10 +752,15 @@ struct pbf_solver {
         for (auto& b : nf4) b.allocate(f4b);
         for (auto& b : nids) b.allocate(u4b);
         for (auto& b : norg) b.allocate(u4b);
-        DeviceBuffer nkeys(u4b), nskeys(u4b), nsidx(u4b), nakeys(u4b), naidx(u4b);
-        DeviceBuffer nbins;
-        if (bins_apply(max_particles, ncells))
+        // The rebuilds' counting sort, or the radix sort's buffers.
+        DeviceBuffer nkeys(u4b), nakeys(u4b), naidx(u4b), nbins, nskeys, nsidx, nscr;
+        if (bins_apply(max_particles, ncells)) {
             nbins.allocate(bin_count_words(ncells) * sizeof(uint32_t));
+        } else {
+            nskeys.allocate(u4b);
+            nsidx.allocate(u4b);
+            nscr.allocate(sort_scratch_bytes(int(max_particles)));
+        }
         DeviceBuffer nfirst((ncells + 1) * sizeof(int));
         DeviceBuffer nsoa(3 * soa_stride_for(max_particles) * sizeof(float));
         DeviceBuffer nnbr((lcap > 0 ? lcap : strd * size_t(maxnb)) * sizeof(uint32_t));
@@ -764,7 +769,7 @@ struct pbf_solver {
             nnboff.allocate((max_particles + 1) * sizeof(uint32_t));
             nnbscr.allocate(nb_scan_scratch_words(max_particles) * sizeof(uint32_t));
         }
-        DeviceBuffer ncnt(u4b), nlam(u4b), nscr(sort_scratch_bytes(int(max_particles)));
+        DeviceBuffer ncnt(u4b), nlam(u4b);
         DeviceBuffer nstat(sizeof(unsigned)), ntmp(f4b);
 
         clear_graphs();
