@@ -236,6 +236,16 @@ void launch_bin_gather(const CellBins& b, const uint32_t* list, const uint32_t* 
                        const uint32_t* org_in, uint32_t* org_out, uint32_t* perm, float* sx,
                        float* sy, float* sz, int n, const unsigned* status, cudaStream_t st);
 
+// The grid build alone, by the same counting sort, for n <= 262,144 positions
+// in device arrays (bins_apply(n, cells)): sorted keys and indices, cell ranges
+// with -1 for empty cells.  keys, place, list: n words each; scratch:
+// bin_grid_words(cells).
+size_t bin_grid_words(uint64_t cells);
+void launch_bin_grid(const float4* pos, int n, const GridConst& g, uint64_t cells,
+                     uint32_t* sorted_keys, uint32_t* sorted_idx, int* cell_start, int* cell_end,
+                     uint32_t* keys, uint32_t* place, uint32_t* list, uint32_t* scratch,
+                     cudaStream_t st);
+
 // --- stable LSD radix sort of (key, index) pairs (pbf_sort.cu) ---------------
 struct SortPlan {
     int n = 0;
