@@ -190,41 +190,48 @@ __device__ __forceinline__ void lambda_add2(const KernelConst& k, LambdaAcc& a, 
     a.gz = fadd(fadd(a.gz, z0), z1);
 }
 
-// Bits of a 32-candidate chunk from j0 that belong to the row range [s, e),
-// less the particle i itself.
+// Bits of a 32-candidate chunk from j0 (the highest: candidate j0) that belong
+// to the row range [s, e), less the particle i itself.
 __device__ __forceinline__ uint32_t chunk_valid(int j0, int s, int e, int i) {
     const int left = e - j0;
-    uint32_t valid = left >= 32 ? 0xffffffffu : ((1u << left) - 1u);
-    if (j0 < s) valid &= ~((1u << (s - j0)) - 1u);
+    uint32_t valid = left >= 32 ? 0xffffffffu : ~(0xffffffffu >> left);
+    if (j0 < s) valid &= 0xffffffffu >> (s - j0);
     const int self = i - j0;
-    if (self >= 0 && self < 32) valid &= ~(1u << self);
+    if (self >= 0 && self < 32) valid &= ~(0x80000000u >> self);
     return valid;
 }
 
-// The neighbour walk of particle i (position pi): writes the list slot-major
-// at out[slot * stride] (at most cap entries) and returns the full count.
-// STORE = false counts the hits without writing the list.
-template <bool B, bool STORE = true>
-__device__ __forceinline__ int walk(const StepConst& c, int i, float4 pi,
-                                    const float* __restrict__ sx, const float* __restrict__ sy,
-                                    const float* __restrict__ sz, const int* __restrict__ first,
-                                    uint32_t* __restrict__ out, int cap) {
+// The hits of particle i (position pi) chunk by chunk, in list order:
+// hits(j0, bits) for each 32-candidate chunk from j0 (the highest bit is
+// candidate j0).
+//
+// Rows z -> y, each one index range walked in ascending order -- exactly the
+// reference's z -> y -> x cell walk (neighbors.cu:52-86).  Each range is
+// tested in 32-candidate chunks from a multiple of 4; candidates outside [s, e)
+// and the particle itself are masked off.  The component arrays are padded
+// (soa_stride_for), so a chunk may read past the last particle.  All lanes of
+// the warp take every row and chunk step together (active: the lane has a
+// particle), and hits is called by all of them.
+template <bool B, class Hits>
+__device__ __forceinline__ void for_each_chunk(const StepConst& c, int i, bool active, float4 pi,
+                                               const float* __restrict__ sx,
+                                               const float* __restrict__ sy,
+                                               const float* __restrict__ sz,
+                                               const int* __restrict__ first, Hits hits) {
     const StencilRows<B> rows(c, i, pi);
     // The hit test d2 <= h2 as a sign bit: for finite d2 it holds exactly
     // when d2 - h2u < 0, h2u being the float just above h2 (the difference
     // of two distinct floats is never zero, and +inf or NaN, the canonical
     // NaN of the FP32 units, give a clear sign bit: no hit, as d2 <= h2).
     const f32x2 h2u = splat2(__uint_as_float(__float_as_uint(c.k.h2) + 1u));
-    const size_t stride = nb_step(c);
     const f32x2 px = splat2(pi.x), py = splat2(pi.y), pz = splat2(pi.z);
-    int count = 0;
-    // 16 candidates from j (a multiple of 4): the x, y, z arrays are read
+    // 8 candidates from j (a multiple of 4): the x, y, z arrays are read
     // four floats at a time and tested two at a time with FP32x2
     // arithmetic; each test's sign bit is shifted into acc (the first
     // candidate ends up highest).
-    auto test16 = [&](int j, uint32_t& acc) {
+    auto test8 = [&](int j, uint32_t& acc) {
 #pragma unroll
-        for (int q = 0; q < 16; q += 4) {
+        for (int q = 0; q < 8; q += 4) {
             const float4 X = __ldg(reinterpret_cast<const float4*>(sx + j + q));
             const float4 Y = __ldg(reinterpret_cast<const float4*>(sy + j + q));
             const float4 Z = __ldg(reinterpret_cast<const float4*>(sz + j + q));
@@ -241,91 +248,114 @@ __device__ __forceinline__ int walk(const StepConst& c, int i, float4 pi,
             acc = __funnelshift_l(__float_as_uint(b1), acc, 1);
         }
     };
-    // Rows z -> y, each one index range walked in ascending order -- exactly
-    // the reference's z -> y -> x cell walk (neighbors.cu:52-86).  Each range
-    // is tested in 32-candidate chunks from a multiple of 4 (the second half
-    // of a chunk only if the range reaches it); candidates outside [s, e) and
-    // the particle itself are masked off, and the hits are then appended in
-    // ascending order.  The component arrays are padded (soa_stride_for), so
-    // a chunk may read past the last particle.
-    for (int z = rows.z0; z <= rows.z1; ++z)
-        for (int y = rows.y0; y <= rows.y1; ++y) {
-            int s, e;
-            if (!rows.range(first, z, y, s, e)) continue;
-            for (int j0 = s & ~3; j0 < e; j0 += 32) {
+    const int R = __reduce_max_sync(0xffffffffu, rows.g.radius);  // of the warp's scenes
+    for (int dz = -R; dz <= R; ++dz)
+        for (int dy = -R; dy <= R; ++dy) {
+            const int z = rows.cz + dz, y = rows.cy + dy;
+            int s = 0, e = 0;
+            if (!active || z < rows.z0 || z > rows.z1 || y < rows.y0 || y > rows.y1 ||
+                !rows.range(first, z, y, s, e))
+                s = e = 0;
+            for (int j0 = s & ~3; __any_sync(0xffffffffu, j0 < e); j0 += 32) {
+                // 8 candidates at a time, as far as the range reaches (with 16
+                // at a time steps took 2 to 4 % longer).
+                const int left = e - j0;
                 uint32_t acc = 0u;
-                test16(j0, acc);
-                if (e - j0 > 16) test16(j0 + 16, acc);
-                else acc <<= 16;
-                uint32_t mask = __brev(acc) & chunk_valid(j0, s, e, i);
-                if constexpr (STORE) {
-                    while (mask) {
-                        const int b = __ffs(mask) - 1;
-                        mask &= mask - 1u;
-                        if (count < cap)
-                            out[static_cast<size_t>(count) * stride] =
-                                static_cast<uint32_t>(j0 + b);
-                        ++count;
+                if (left > 0) {
+                    test8(j0, acc);
+                    if (left <= 8) {
+                        acc <<= 24;
+                    } else {
+                        test8(j0 + 8, acc);
+                        if (left <= 16) {
+                            acc <<= 16;
+                        } else {
+                            test8(j0 + 16, acc);
+                            if (left <= 24) acc <<= 8;
+                            else test8(j0 + 24, acc);
+                        }
                     }
-                } else {
-                    count += __popc(mask);
+                    acc &= chunk_valid(j0, s, e, i);
                 }
+                hits(j0, acc);
             }
         }
-    return count;
 }
 
-// Second pass over the list just written: the constraint terms run once per
-// neighbour instead of once per candidate in which any lane of the warp hit.
-// Same order as the list, so the same sums.  Neighbours are taken two at a
-// time with FP32x2 arithmetic; the sums stay in list order.  The next pair's
-// indices are loaded before this pair is gathered.
-template <bool B>
-__device__ __forceinline__ float lambda_of_list(const StepConst& c, int i, float4 pi,
-                                                const float4* __restrict__ xs,
-                                                const uint32_t* __restrict__ out, size_t stride,
-                                                int count) {
-    const f32x2 px = pack2(pi.x, pi.x), py = pack2(pi.y, pi.y), pz = pack2(pi.z, pi.z);
-    LambdaAcc acc{c.k.c_poly6, 0.0f, 0.0f, 0.0f, 0.0f};
-    int k = 0;
-    uint32_t na = 0u, nb2 = 0u;
-    if (count >= 2) {
-        na = out[0];
-        nb2 = out[stride];
-    }
-    for (; k + 2 <= count; k += 2) {
-        const uint32_t ja = na, jb = nb2;
-        if (k + 4 <= count) {
-            na = out[static_cast<size_t>(k + 2) * stride];
-            nb2 = out[static_cast<size_t>(k + 3) * stride];
+// Entries of a lane's queue of chunks with hits (8 bytes each, in shared
+// memory).  A stencil of nine rows with some 20 candidates each has 9 to 11 such
+// chunks; search time at 10 / 12 / 16 entries: 0.930 / 0.923 / 0.928 ms at
+// 1,048,576 particles, 10.56 / 10.41 / 10.42 for 8,388,608 in dense blobs.
+constexpr int kQueue = 12;
+inline size_t queue_bytes(int threads) { return sizeof(uint2) * kQueue * threads; }
+
+// The neighbour walk of particle i with the terms of its neighbours: writes the
+// list slot-major at out[slot * stride] (at most cap entries), hands the
+// neighbours over in list order (load, use2, use1 as for
+// for_each_neighbor_pair) and returns the full count.
+//
+// Bound by instruction issue.  Appending the hits of each chunk at once costs a
+// warp the largest number of hits of any lane, chunk by chunk (2 to 3 times the
+// average), and the terms need a second pass over the list.  So the chunks with
+// hits are queued, and the lanes take their neighbours from their queues one by
+// one, in step: list entry and terms in one loop whose length is the largest
+// neighbour count.  The queues are emptied together when any is full (lanes that
+// empty theirs by themselves: walk 30 to 80 % longer in dense scenes).  Walk and
+// lambda, before and after: 38 -> 29 us at 65,536 particles, 76 -> 63 at
+// 262,144, 280 -> 222 at 1,048,576 and 875 -> 720 for 256 batched scenes; the
+// final walk with XSPH at 1,048,576 310 -> 254 (72 registers; 64 spill: 281).
+template <bool B, class T, class Load, class Use2, class Use1>
+__device__ __forceinline__ int walk_terms(const StepConst& c, int i, bool active, float4 pi,
+                                          const float* __restrict__ sx,
+                                          const float* __restrict__ sy,
+                                          const float* __restrict__ sz,
+                                          const int* __restrict__ first,
+                                          uint32_t* __restrict__ out, int cap, Load load,
+                                          Use2 use2, Use1 use1) {
+    extern __shared__ uint2 queues[];
+    uint2* const queue = queues + threadIdx.x;
+    const int step = blockDim.x;
+    const size_t stride = nb_step(c);
+    int count = 0;         // neighbours handed over
+    int found = 0;         // neighbours in the queue
+    uint2* tail = queue;
+    const uint2* const end_of_queue = queue + kQueue * step;
+    auto drain = [&]() {
+        const uint2* head = queue;
+        uint32_t bits = 0u, j0 = 0u;
+        auto pop = [&]() {
+            if (!bits) {
+                const uint2 q = *head;
+                head += step;
+                j0 = q.x;
+                bits = q.y;
+            }
+            const int b = __clz(bits);
+            bits &= ~(0x80000000u >> b);
+            const uint32_t j = j0 + b;
+            if (count < cap) out[static_cast<size_t>(count) * stride] = j;
+            ++count;
+            return j;
+        };
+        const int end = count + found;
+        while (count + 2 <= end) {
+            const T a = load(pop()), b = load(pop());
+            use2(a, b);
         }
-        const float4 a = __ldg(&xs[ja]);
-        const float4 b = __ldg(&xs[jb]);
-        const f32x2 dx = sub2(px, pack2(a.x, b.x));
-        const f32x2 dy = sub2(py, pack2(a.y, b.y));
-        const f32x2 dz = sub2(pz, pack2(a.z, b.z));
-        lambda_add2(c.k, acc, dx, dy, dz, dist2x2(dx, dy, dz));
-    }
-    if (k < count) {
-        const float4 pj = __ldg(&xs[out[static_cast<size_t>(k) * stride]]);
-        const float dx = fsub(pi.x, pj.x), dy = fsub(pi.y, pj.y), dz = fsub(pi.z, pj.z);
-        lambda_add(c.k, acc, dx, dy, dz, dist2(dx, dy, dz));
-    }
-    return lambda_of_acc<B>(c, i, acc);
-}
-
-// What k_search does once particle i's list (count entries) is written.
-template <bool LAMBDA, bool B>
-__device__ __forceinline__ void search_tail(const StepConst& c, int i, float4 pi,
-                                            const float4* __restrict__ xs,
-                                            const uint32_t* __restrict__ out, int count,
-                                            int* __restrict__ cnt, float* __restrict__ lam,
-                                            unsigned* __restrict__ status) {
-    cnt[i] = count;
-    if (count > c.max_nb) atomicOr(status, kStatusNeighborOverflow);
-    if (LAMBDA)
-        lam[i] = count > c.max_nb ? CUDART_NAN_F
-                                  : lambda_of_list<B>(c, i, pi, xs, out, nb_step(c), count);
+        if (count < end) use1(load(pop()));
+        tail = queue;
+        found = 0;
+    };
+    for_each_chunk<B>(c, i, active, pi, sx, sy, sz, first, [&](int j0, uint32_t bits) {
+        if (bits) {
+            *tail = make_uint2(static_cast<uint32_t>(j0), bits);
+            tail += step;
+            found += __popc(bits);
+        }
+        if (__any_sync(0xffffffffu, tail == end_of_queue)) drain();
+    });
+    drain();
+    return count;
 }
 
 template <bool LAMBDA, bool B>
@@ -334,12 +364,32 @@ k_search(const float4* __restrict__ xs, const float* __restrict__ sx,
          const float* __restrict__ sy, const float* __restrict__ sz, const int* __restrict__ first,
          StepConst c, int n, uint32_t* __restrict__ nbr, int* __restrict__ cnt,
          float* __restrict__ lam, unsigned* __restrict__ status) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || fatal(status)) return;
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (__any_sync(0xffffffffu, fatal(status))) return;
+    const bool active = i < n;
+    i = min(i, n - 1);
     const float4 pi = xs[i];
-    uint32_t* __restrict__ out = nbr + nb_first(c, i);
-    const int count = walk<B>(c, i, pi, sx, sy, sz, first, out, c.max_nb);
-    search_tail<LAMBDA, B>(c, i, pi, xs, out, count, cnt, lam, status);
+    const f32x2 px = splat2(pi.x), py = splat2(pi.y), pz = splat2(pi.z);
+    LambdaAcc acc{c.k.c_poly6, 0.0f, 0.0f, 0.0f, 0.0f};
+    const int count = walk_terms<B, float4>(
+        c, i, active, pi, sx, sy, sz, first, nbr + nb_first(c, i), c.max_nb,
+        [&](uint32_t j) { return LAMBDA ? __ldg(&xs[j]) : float4{}; },
+        [&](const float4& a, const float4& b) {
+            if (!LAMBDA) return;
+            const f32x2 dx = sub2(px, pack2(a.x, b.x));
+            const f32x2 dy = sub2(py, pack2(a.y, b.y));
+            const f32x2 dz = sub2(pz, pack2(a.z, b.z));
+            lambda_add2(c.k, acc, dx, dy, dz, dist2x2(dx, dy, dz));
+        },
+        [&](const float4& a) {
+            if (!LAMBDA) return;
+            const float dx = fsub(pi.x, a.x), dy = fsub(pi.y, a.y), dz = fsub(pi.z, a.z);
+            lambda_add(c.k, acc, dx, dy, dz, dist2(dx, dy, dz));
+        });
+    if (!active) return;
+    cnt[i] = count;
+    if (count > c.max_nb) atomicOr(status, kStatusNeighborOverflow);
+    if (LAMBDA) lam[i] = count > c.max_nb ? CUDART_NAN_F : lambda_of_acc<B>(c, i, acc);
 }
 
 // Compact lists, first pass: the walk's neighbour count only.
@@ -349,9 +399,14 @@ k_count(const float4* __restrict__ xs, const float* __restrict__ sx,
         const float* __restrict__ sy, const float* __restrict__ sz,
         const int* __restrict__ first, StepConst c, int n, int* __restrict__ cnt,
         unsigned* __restrict__ status) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || fatal(status)) return;
-    const int count = walk<B, false>(c, i, xs[i], sx, sy, sz, first, nullptr, c.max_nb);
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (__any_sync(0xffffffffu, fatal(status))) return;
+    const bool active = i < n;
+    i = min(i, n - 1);
+    int count = 0;
+    for_each_chunk<B>(c, i, active, xs[i], sx, sy, sz, first,
+                      [&](int, uint32_t bits) { count += __popc(bits); });
+    if (!active) return;
     cnt[i] = count;
     if (count > c.max_nb) atomicOr(status, kStatusNeighborOverflow);
 }
@@ -654,6 +709,34 @@ k_finalize(const uint32_t* __restrict__ org, const float4* __restrict__ x_old,
 }
 
 // applyXsphViscosity (pbf_solver_kernels.cu:213-266).
+struct XsphAcc {
+    float x, y, z;
+};
+__device__ __forceinline__ void xsph_add2(const KernelConst& k, XsphAcc& s, float4 pi, float4 vi,
+                                          const PosVel& a, const PosVel& b) {
+    float w0, w1, x0, x1, y0, y1, z0, z1;
+    unpack2(poly6_2(k, dist2x2(diff2(pi.x, a.p.x, b.p.x), diff2(pi.y, a.p.y, b.p.y),
+                               diff2(pi.z, a.p.z, b.p.z))),
+            w0, w1);
+    unpack2(rdiff2(a.v.x, b.v.x, vi.x), x0, x1);
+    unpack2(rdiff2(a.v.y, b.v.y, vi.y), y0, y1);
+    unpack2(rdiff2(a.v.z, b.v.z, vi.z), z0, z1);
+    s.x = ffma(x1, w1, ffma(x0, w0, s.x));
+    s.y = ffma(y1, w1, ffma(y0, w0, s.y));
+    s.z = ffma(z1, w1, ffma(z0, w0, s.z));
+}
+__device__ __forceinline__ void xsph_add(const KernelConst& k, XsphAcc& s, float4 pi, float4 vi,
+                                         const PosVel& q) {
+    const float w = poly6(k, dist2(fsub(pi.x, q.p.x), fsub(pi.y, q.p.y), fsub(pi.z, q.p.z)));
+    s.x = ffma(fsub(q.v.x, vi.x), w, s.x);
+    s.y = ffma(fsub(q.v.y, vi.y), w, s.y);
+    s.z = ffma(fsub(q.v.z, vi.z), w, s.z);
+}
+__device__ __forceinline__ float4 xsph_finish(float xsph_c, const XsphAcc& s, float4 vi) {
+    return make_float4(ffma(xsph_c, s.x, vi.x), ffma(xsph_c, s.y, vi.y), ffma(xsph_c, s.z, vi.z),
+                       vi.w);
+}
+
 __device__ __forceinline__ float4 xsph_one(const StepConst& c, const float4* __restrict__ x,
                                            const float4* __restrict__ v,
                                            const uint32_t* __restrict__ nbr, int count, int i,
@@ -662,31 +745,13 @@ __device__ __forceinline__ float4 xsph_one(const StepConst& c, const float4* __r
     if (!count_ok(count, c.max_nb))
         return make_float4(CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F, vi.w);
     const float4 pi = x[i];
-    float cx = 0.0f, cy = 0.0f, cz = 0.0f;
+    XsphAcc s{0.0f, 0.0f, 0.0f};
     for_each_neighbor_pair<PosVel>(
         nbr + nb_first(c, i), nb_step(c), count,
         [&](uint32_t j) { return PosVel{__ldg(&x[j]), __ldg(&v[j])}; },
-        [&](const PosVel& a, const PosVel& b) {
-            float w0, w1, x0, x1, y0, y1, z0, z1;
-            unpack2(poly6_2(c.k, dist2x2(diff2(pi.x, a.p.x, b.p.x), diff2(pi.y, a.p.y, b.p.y),
-                                         diff2(pi.z, a.p.z, b.p.z))),
-                    w0, w1);
-            unpack2(rdiff2(a.v.x, b.v.x, vi.x), x0, x1);
-            unpack2(rdiff2(a.v.y, b.v.y, vi.y), y0, y1);
-            unpack2(rdiff2(a.v.z, b.v.z, vi.z), z0, z1);
-            cx = ffma(x1, w1, ffma(x0, w0, cx));
-            cy = ffma(y1, w1, ffma(y0, w0, cy));
-            cz = ffma(z1, w1, ffma(z0, w0, cz));
-        },
-        [&](const PosVel& q) {
-            const float w =
-                poly6(c.k, dist2(fsub(pi.x, q.p.x), fsub(pi.y, q.p.y), fsub(pi.z, q.p.z)));
-            cx = ffma(fsub(q.v.x, vi.x), w, cx);
-            cy = ffma(fsub(q.v.y, vi.y), w, cy);
-            cz = ffma(fsub(q.v.z, vi.z), w, cz);
-        });
-    return make_float4(ffma(xsph_c, cx, vi.x), ffma(xsph_c, cy, vi.y), ffma(xsph_c, cz, vi.z),
-                       vi.w);
+        [&](const PosVel& a, const PosVel& b) { xsph_add2(c.k, s, pi, vi, a, b); },
+        [&](const PosVel& q) { xsph_add(c.k, s, pi, vi, q); });
+    return xsph_finish(xsph_c, s, vi);
 }
 
 template <bool B>
@@ -704,40 +769,37 @@ k_xsph(const float4* __restrict__ x, const float4* __restrict__ v,
     v_out[i] = out;
 }
 
-// What the final walk does once particle i's list (count entries) is written.
+// The final rebuild's walk with applyXsphViscosity fused in (velocities v are
+// the updated ones, computed before this walk), and with the velocity response
+// when no vorticity pass follows.
 template <bool B>
-__device__ __forceinline__ void xsph_tail(const StepConst& c, int i, float4 pi,
-                                          const float4* __restrict__ xs,
-                                          const uint32_t* __restrict__ nbr, int count,
-                                          int* __restrict__ cnt, const float4* __restrict__ v,
-                                          float4* __restrict__ v_out,
-                                          const float4* __restrict__ vin, bool resolve,
-                                          unsigned* __restrict__ status) {
-    cnt[i] = count;
-    if (count > c.max_nb) atomicOr(status, kStatusNeighborOverflow);
-    float4 out = xsph_one(c, xs, v, nbr, count, i, B ? scene_of(c, i).xsph_c : c.xsph_c);
-    if (resolve)
-        resolve_velocity(colliders_of<B>(c, i), c.particle_radius, c.restitution, c.friction,
-                         pi, vin[i], out);
-    v_out[i] = out;
-}
-
-// The final rebuild's walk with XSPH fused in: the list is written, then
-// applyXsphViscosity runs over it in a second pass (velocities v are the
-// updated ones, computed before this walk), with the velocity response when
-// no vorticity pass follows.
-template <bool B>
-__global__ void __launch_bounds__(kMaxTunedBlock)
+__global__ void PBF_GATHER_REGS(72)
 k_search_xsph(const float4* __restrict__ xs, const float* __restrict__ sx,
               const float* __restrict__ sy, const float* __restrict__ sz,
               const int* __restrict__ first, StepConst c, int n, uint32_t* __restrict__ nbr,
               int* __restrict__ cnt, const float4* __restrict__ v, float4* __restrict__ v_out,
               const float4* __restrict__ vin, bool resolve, unsigned* __restrict__ status) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || fatal(status)) return;
-    const float4 pi = xs[i];
-    const int count = walk<B>(c, i, pi, sx, sy, sz, first, nbr + nb_first(c, i), c.max_nb);
-    xsph_tail<B>(c, i, pi, xs, nbr, count, cnt, v, v_out, vin, resolve, status);
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (__any_sync(0xffffffffu, fatal(status))) return;
+    const bool active = i < n;
+    i = min(i, n - 1);
+    const float4 pi = xs[i], vi = v[i];
+    XsphAcc s{0.0f, 0.0f, 0.0f};
+    const int count = walk_terms<B, PosVel>(
+        c, i, active, pi, sx, sy, sz, first, nbr + nb_first(c, i), c.max_nb,
+        [&](uint32_t j) { return PosVel{__ldg(&xs[j]), __ldg(&v[j])}; },
+        [&](const PosVel& a, const PosVel& b) { xsph_add2(c.k, s, pi, vi, a, b); },
+        [&](const PosVel& q) { xsph_add(c.k, s, pi, vi, q); });
+    if (!active) return;
+    cnt[i] = count;
+    if (count > c.max_nb) atomicOr(status, kStatusNeighborOverflow);
+    float4 out = count > c.max_nb
+                     ? make_float4(CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F, vi.w)
+                     : xsph_finish(B ? scene_of(c, i).xsph_c : c.xsph_c, s, vi);
+    if (resolve)
+        resolve_velocity(colliders_of<B>(c, i), c.particle_radius, c.restitution, c.friction,
+                         pi, vin[i], out);
+    v_out[i] = out;
 }
 
 // computeVorticity (pbf_solver_kernels.cu:268-315).
@@ -1048,16 +1110,16 @@ void launch_search(const float4* xs, const float* sx, const float* sy, const flo
     }
     const unsigned g = blocks_for(n, bs);
     if (with_lambda && c.scenes)
-        launch_k(k_search<true, true>, g, bs, st, xs, sx, sy, sz, first, c, n, nbr, cnt, lam,
+        launch_k_smem(k_search<true, true>, g, bs, queue_bytes(bs), st, xs, sx, sy, sz, first, c, n, nbr, cnt, lam,
                  status);
     else if (with_lambda)
-        launch_k(k_search<true, false>, g, bs, st, xs, sx, sy, sz, first, c, n, nbr, cnt, lam,
+        launch_k_smem(k_search<true, false>, g, bs, queue_bytes(bs), st, xs, sx, sy, sz, first, c, n, nbr, cnt, lam,
                  status);
     else if (c.scenes)
-        launch_k(k_search<false, true>, g, bs, st, xs, sx, sy, sz, first, c, n, nbr, cnt, lam,
+        launch_k_smem(k_search<false, true>, g, bs, queue_bytes(bs), st, xs, sx, sy, sz, first, c, n, nbr, cnt, lam,
                  status);
     else
-        launch_k(k_search<false, false>, g, bs, st, xs, sx, sy, sz, first, c, n, nbr, cnt, lam,
+        launch_k_smem(k_search<false, false>, g, bs, queue_bytes(bs), st, xs, sx, sy, sz, first, c, n, nbr, cnt, lam,
                  status);
 }
 
@@ -1073,10 +1135,10 @@ void launch_search_xsph(const float4* xs, const float* sx, const float* sy, cons
     }
     const unsigned g = blocks_for(n, bs);
     if (c.scenes)
-        launch_k(k_search_xsph<true>, g, bs, st, xs, sx, sy, sz, first, c, n, nbr, cnt, v, v_out,
+        launch_k_smem(k_search_xsph<true>, g, bs, queue_bytes(bs), st, xs, sx, sy, sz, first, c, n, nbr, cnt, v, v_out,
                  vin, resolve, status);
     else
-        launch_k(k_search_xsph<false>, g, bs, st, xs, sx, sy, sz, first, c, n, nbr, cnt, v, v_out,
+        launch_k_smem(k_search_xsph<false>, g, bs, queue_bytes(bs), st, xs, sx, sy, sz, first, c, n, nbr, cnt, v, v_out,
                  vin, resolve, status);
 }
 
