@@ -1072,27 +1072,26 @@ inline int group_lanes(const StepConst& c, int n) {
 
 // Threads per block of the neighbour kernels by default.  Smaller blocks even
 // out the last wave once there are several blocks an SM: frame at 256 / 128 /
-// 64 threads 302 / 288 / 289 us at 65,536 particles, 414 / 388 / 382 at 131,072,
-// 708 / 687 / 685 at 262,144, 2,389 / 2,331 / 2,349 at 1,048,576; 242 / 248 /
-// 248 at 32,768, and 7.47 / 7.60 / 7.69 ms for 256 batched scenes.
+// 64 threads 358 / 329 / 331 us at 131,072 particles, 608 / 593 / 598 at
+// 262,144, 1,837 / 1,806 / 1,829 at 1,048,576, 6.70 / 6.66 / 6.68 ms for 256
+// batched scenes; 242 / 242 / 241 at 65,536 and 202 / 210 / 215 at 32,768.
 constexpr size_t kBlock128From = 57344;
-int default_block(size_t n, int lanes, bool batched) {
+int default_block(size_t n, int lanes) {
     if (lanes > 1) return kGroupBlock;
-    return n >= kBlock128From && !batched ? 128 : kBlock;
+    return n >= kBlock128From ? 128 : kBlock;
 }
 inline int tuned_block(const StepConst& c, int n, int k) {
-    return c.blk[k] > 0 ? c.blk[k] : default_block(n, group_lanes(c, n), c.scenes != nullptr);
+    return c.blk[k] > 0 ? c.blk[k] : default_block(n, group_lanes(c, n));
 }
 
 // Lanes per particle of the neighbour kernels by default (the walks take nine,
 // a stencil row each, from 2 on).  Fewer lanes do less work in all, more make
-// a shorter launch.  Measured steps of dam breaks in motion at 1 / 8 / 16 / 32
-// lanes: 162 / 98 / 92 / 88 us at 1,024 particles, 190 / 108 / 103 / 99 at
-// 2,048, 197 / 115 / 109 / 109 at 4,096, 206 / 131 / 128 / 144 at 8,192, 222 /
-// 165 / 173 / 193 at 13,824, 228 / 178 / 192 / 214 at 16,384, 231 / 235 / 252 /
-// 287 at 24,576 and 236 / 281 / 296 / 340 at 32,768 (three lanes with a plane
-// of rows each for the walk: 225 at 24,576, 250 at 32,768).
-constexpr size_t kLanes32Max = 3072, kLanes16Max = 10240, kLanes8Max = 22528;
+// a shorter launch.  Measured steps of dam breaks in motion at 8 / 16 / 32
+// lanes: 98 / 92 / 88 us at 1,024 particles, 108 / 103 / 99 at 2,048, 115 / 109
+// / 109 at 4,096, 131 / 128 / 144 at 8,192, 165 / 173 / 193 at 13,824; at 1 / 8
+// lanes 178 / 119 at 6,144, 202 / 168 at 13,824, 208 / 177 at 16,384, 200 / 207
+// at 20,480 and 194 / 228 at 24,576.
+constexpr size_t kLanes32Max = 3072, kLanes16Max = 10240, kLanes8Max = 18432;
 
 int default_walk_lanes(size_t n, int max_nb) {
     int L = n <= kLanes32Max ? 32 : (n <= kLanes16Max ? 16 : (n <= kLanes8Max ? 8 : 1));

@@ -61,7 +61,7 @@ struct StepConst {
 // (slot-major lists with max_nb slots).
 int default_walk_lanes(size_t n, int max_nb);
 // Threads per block of the neighbour kernels that no tuning has set.
-int default_block(size_t n, int lanes, bool batched);
+int default_block(size_t n, int lanes);
 
 // Stride (floats) of the x, y, z component arrays the walks read, for n
 // particles: a multiple of 64 (every array 256-byte aligned, so the walk's

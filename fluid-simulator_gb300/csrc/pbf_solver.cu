@@ -1253,7 +1253,7 @@ pbf_status pbf_block_sizes(const pbf_solver* s, int* sizes, int count) {
     }
     for (int k = 0; k < count && k < kTunedCount; ++k)
         sizes[k] = s->tuned[k] > 0 ? s->tuned[k]
-                                   : default_block(s->n, s->walk_lanes(), s->nscenes > 0);
+                                   : default_block(s->n, s->walk_lanes());
     return PBF_OK;
 }
 

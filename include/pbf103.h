@@ -170,7 +170,7 @@ pbf_status pbf_block_sizes(const pbf_solver* s, int* sizes, int count);
  * else 1,024 below 2^19 particles and 4,096 from there on). */
 pbf_status pbf_sort_tile(const pbf_solver* s, int* keys_per_tile);
 /* Lanes per particle of the list-writing walks in use: the value set by
- * pbf_set_walk_lanes, else 8 (also where small scenes take more) up to 22,528
+ * pbf_set_walk_lanes, else 8 (also where small scenes take more) up to 18,432
  * particles and 1 from there on (always 1 with compact lists; at most
  * max_neighbors). */
 pbf_status pbf_walk_lanes(const pbf_solver* s, int* lanes);

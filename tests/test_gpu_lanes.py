@@ -1,6 +1,6 @@
 """The lane-group kernels at the sizes and lengths where they change.
 
-Groups of 32, 16 and 8 lanes by default up to 3,072, 10,240 and 22,528
+Groups of 32, 16 and 8 lanes by default up to 3,072, 10,240 and 18,432
 particles, one thread per particle above, and 2, 4 or 8 when set; walks of
 nine lanes with three particles a warp.  A packed core (rows of more than 32
 and more than 64 candidates, lists longer than a 64-entry stash) inside a
@@ -12,7 +12,8 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [(n, 0) for n in (1, 2, 3, 4, 31, 97, 3072, 3073, 10240, 10241, 22528, 22529)]
+SIZES = [(n, 0) for n in (1, 2, 3, 4, 31, 97, 3072, 3073, 10240, 10241, 18432, 18433, 22528,
+                         22529)]
 SIZES += [(n, lanes) for lanes in (2, 4, 8) for n in (1, 5, 1000)]
 
 
