@@ -282,6 +282,57 @@ __device__ __forceinline__ void for_each_chunk(const StepConst& c, int i, bool a
         }
 }
 
+// Compact lists.  The lists of a warp's 32 particles share a slice as wide as
+// the longest of them, entry after entry (offset 32 w + lane, step 32): the 32
+// threads that read entry k of their lists read 128 bytes in a row, as with
+// slot-major lists.  Back to back (step 1) they read 32 sectors: delta p 148
+// against 98 us, vorticity 188 against 137, confinement 170 against 123 at
+// 1,048,576 particles.  The walks take the slices one after another as they go
+// (c.nb_ctl counts the entries), so that no pass has to count the neighbours
+// first: frame 17.96 ms with a walk that counts and a scan before each walk,
+// 13.84 without, at 8,388,608 particles; 2.37 and 1.78 at 1,048,576.  The slices
+// of the scenes here take a tenth to a third more entries than the lists.  When
+// they do not fit, the rebuild starts over: counts, a scan of them, and the walk
+// into lists back to back (or in slices where those fit after all); the frame's
+// later rebuilds then go that way at once (1,048,576 particles 3.00 ms with 4 %
+// more capacity than the lists take).
+constexpr size_t kNoPlace = ~size_t(0);
+constexpr int kCtlUsed = 0, kCtlFailed = 2, kCtlScanned = 3;  // words of c.nb_ctl
+
+// The first entry of the lane's list, in a slice for the longest of the warp's.
+__device__ __forceinline__ size_t alloc_lists(const StepConst& c, int count) {
+    const int lane = threadIdx.x & 31;
+    const unsigned need = 32u * __reduce_max_sync(0xffffffffu, static_cast<unsigned>(count));
+    unsigned long long at = 0ull;
+    if (lane == 0)
+        at = atomicAdd(reinterpret_cast<unsigned long long*>(c.nb_ctl + kCtlUsed),
+                       static_cast<unsigned long long>(need));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (at + need > c.nb_cap) {
+        if (lane == 0) c.nb_ctl[kCtlFailed] = 1u;
+        return kNoPlace;
+    }
+    return static_cast<size_t>(at) + lane;
+}
+
+// Whether the walk that allocates does nothing; thread 0 of the grid sets the
+// slices' step.
+__device__ __forceinline__ bool skip_alloc(const StepConst& c) {
+    const bool skip = !c.nb_retry && __ldcg(&c.nb_ctl[kCtlScanned]) != 0u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (skip) c.nb_ctl[kCtlFailed] = 1u;
+        else *c.nb_step = 32u;
+    }
+    return skip;
+}
+
+// Whether the walk into scanned offsets does nothing.
+__device__ __forceinline__ bool skip_scanned(const StepConst& c) {
+    if (c.nb_off == nullptr) return false;  // slot-major lists
+    if (blockIdx.x == 0 && threadIdx.x == 0) c.nb_ctl[kCtlFailed] = 0u;
+    return __ldcg(&c.nb_ctl[kCtlScanned]) == 0u;
+}
+
 // Entries of a lane's queue of chunks with hits (8 bytes each, in shared
 // memory).  A stencil of nine rows with some 20 candidates each has 9 to 11 such
 // chunks; search time at 10 / 12 / 16 entries: 0.930 / 0.923 / 0.928 ms at
@@ -290,9 +341,11 @@ constexpr int kQueue = 12;
 inline size_t queue_bytes(int threads) { return sizeof(uint2) * kQueue * threads; }
 
 // The neighbour walk of particle i with the terms of its neighbours: writes the
-// list slot-major at out[slot * stride] (at most cap entries), hands the
-// neighbours over in list order (load, use2, use1 as for
-// for_each_neighbor_pair) and returns the full count.
+// list into nbr (at most cap entries), hands the neighbours over in list order
+// (load, use2, use1 as for for_each_neighbor_pair) and returns the full count.
+// ALLOC: the warp takes the place of its lists (see alloc_lists) once it knows
+// their lengths, in the first walk when the queues held all hits, else before a
+// second; -1 if there is no place left.
 //
 // Bound by instruction issue.  Appending the hits of each chunk at once costs a
 // warp the largest number of hits of any lane, chunk by chunk (2 to 3 times the
@@ -304,18 +357,21 @@ inline size_t queue_bytes(int threads) { return sizeof(uint2) * kQueue * threads
 // lambda, before and after: 38 -> 29 us at 65,536 particles, 76 -> 63 at
 // 262,144, 280 -> 222 at 1,048,576 and 875 -> 720 for 256 batched scenes; the
 // final walk with XSPH at 1,048,576 310 -> 254 (72 registers; 64 spill: 281).
-template <bool B, class T, class Load, class Use2, class Use1>
+template <bool B, bool ALLOC, class T, class Load, class Use2, class Use1>
 __device__ __forceinline__ int walk_terms(const StepConst& c, int i, bool active, float4 pi,
                                           const float* __restrict__ sx,
                                           const float* __restrict__ sy,
                                           const float* __restrict__ sz,
                                           const int* __restrict__ first,
-                                          uint32_t* __restrict__ out, int cap, Load load,
+                                          uint32_t* __restrict__ nbr, int cap, Load load,
                                           Use2 use2, Use1 use1) {
     extern __shared__ uint2 queues[];
     uint2* const queue = queues + threadIdx.x;
     const int step = blockDim.x;
-    const size_t stride = nb_step(c);
+    uint32_t* __restrict__ out = ALLOC ? nbr : nbr + nb_first(c, i);
+    const size_t stride = ALLOC ? 32 : nb_step(c);
+    bool placed = !ALLOC;  // out is known
+    bool over = false;     // hits left out of the queue
     int count = 0;         // neighbours handed over
     int found = 0;         // neighbours in the queue
     uint2* tail = queue;
@@ -346,19 +402,35 @@ __device__ __forceinline__ int walk_terms(const StepConst& c, int i, bool active
         tail = queue;
         found = 0;
     };
-    for_each_chunk<B>(c, i, active, pi, sx, sy, sz, first, [&](int j0, uint32_t bits) {
-        if (bits) {
-            *tail = make_uint2(static_cast<uint32_t>(j0), bits);
-            tail += step;
-            found += __popc(bits);
-        }
-        if (__any_sync(0xffffffffu, tail == end_of_queue)) drain();
-    });
+#pragma unroll 1
+    for (;;) {
+        for_each_chunk<B>(c, i, active, pi, sx, sy, sz, first, [&](int j0, uint32_t bits) {
+            if (bits) {
+                if (!ALLOC || tail != end_of_queue) {
+                    *tail = make_uint2(static_cast<uint32_t>(j0), bits);
+                    tail += step;
+                } else {
+                    over = true;
+                }
+                found += __popc(bits);
+            }
+            if (placed && __any_sync(0xffffffffu, tail == end_of_queue)) drain();
+        });
+        if (placed) break;
+        const size_t at = alloc_lists(c, min(found, cap));
+        if (at == kNoPlace) return -1;
+        out = nbr + at;
+        if (active) c.nb_off[i] = static_cast<uint32_t>(at);
+        placed = true;
+        if (!__any_sync(0xffffffffu, over)) break;
+        tail = queue;
+        found = 0;
+    }
     drain();
     return count;
 }
 
-template <bool LAMBDA, bool B>
+template <bool LAMBDA, bool B, bool ALLOC>
 __global__ void __launch_bounds__(kMaxTunedBlock)
 k_search(const float4* __restrict__ xs, const float* __restrict__ sx,
          const float* __restrict__ sy, const float* __restrict__ sz, const int* __restrict__ first,
@@ -366,13 +438,14 @@ k_search(const float4* __restrict__ xs, const float* __restrict__ sx,
          float* __restrict__ lam, unsigned* __restrict__ status) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (__any_sync(0xffffffffu, fatal(status))) return;
+    if (ALLOC ? skip_alloc(c) : skip_scanned(c)) return;
     const bool active = i < n;
     i = min(i, n - 1);
     const float4 pi = xs[i];
     const f32x2 px = splat2(pi.x), py = splat2(pi.y), pz = splat2(pi.z);
     LambdaAcc acc{c.k.c_poly6, 0.0f, 0.0f, 0.0f, 0.0f};
-    const int count = walk_terms<B, float4>(
-        c, i, active, pi, sx, sy, sz, first, nbr + nb_first(c, i), c.max_nb,
+    const int count = walk_terms<B, ALLOC, float4>(
+        c, i, active, pi, sx, sy, sz, first, nbr, c.max_nb,
         [&](uint32_t j) { return LAMBDA ? __ldg(&xs[j]) : float4{}; },
         [&](const float4& a, const float4& b) {
             if (!LAMBDA) return;
@@ -386,13 +459,13 @@ k_search(const float4* __restrict__ xs, const float* __restrict__ sx,
             const float dx = fsub(pi.x, a.x), dy = fsub(pi.y, a.y), dz = fsub(pi.z, a.z);
             lambda_add(c.k, acc, dx, dy, dz, dist2(dx, dy, dz));
         });
-    if (!active) return;
+    if (!active || count < 0) return;
     cnt[i] = count;
     if (count > c.max_nb) atomicOr(status, kStatusNeighborOverflow);
     if (LAMBDA) lam[i] = count > c.max_nb ? CUDART_NAN_F : lambda_of_acc<B>(c, i, acc);
 }
 
-// Compact lists, first pass: the walk's neighbour count only.
+// Compact lists that start over: the walk's neighbour count only.
 template <bool B>
 __global__ void __launch_bounds__(kMaxTunedBlock)
 k_count(const float4* __restrict__ xs, const float* __restrict__ sx,
@@ -401,6 +474,8 @@ k_count(const float4* __restrict__ xs, const float* __restrict__ sx,
         unsigned* __restrict__ status) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (__any_sync(0xffffffffu, fatal(status))) return;
+    if (i < 2) c.nb_ctl[kCtlUsed + i] = 0u;  // for the next rebuild
+    if (__ldcg(&c.nb_ctl[kCtlFailed]) == 0u) return;
     const bool active = i < n;
     i = min(i, n - 1);
     int count = 0;
@@ -411,18 +486,9 @@ k_count(const float4* __restrict__ xs, const float* __restrict__ sx,
     if (count > c.max_nb) atomicOr(status, kStatusNeighborOverflow);
 }
 
-// Exclusive scan of the counts into list offsets, in three launches: tile
-// totals, a scan of the totals, and the offsets.  64-bit sums; offsets are
-// 32-bit because the list capacity is below 2^32.
-//
-// Where the capacity allows, the lists of 32 consecutive particles share a
-// slice as wide as the longest of them, entry after entry (offsets 32 w + lane,
-// step 32): the 32 threads that read entry k of their lists read 128 bytes in a
-// row, as with slot-major lists.  Back to back (step 1) they read 32 sectors:
-// delta p 148 against 98 us, vorticity 188 against 137, confinement 170 against
-// 123 and walk + lambda 314 against 280 at 1,048,576 particles.  The slices of
-// the scenes here take a tenth to a third more entries than the lists; when they
-// would not fit, the lists go back to back as long as these do.
+// Exclusive scan of the counts into list offsets, in two launches: tile totals,
+// and the offsets.  64-bit sums; offsets are 32-bit because the list capacity is
+// below 2^32.
 constexpr int kScanThreads = 256, kScanItems = 8, kScanTile = kScanThreads * kScanItems;
 
 __device__ __forceinline__ unsigned long long block_scan_u64(unsigned long long v,
@@ -477,9 +543,10 @@ __device__ __forceinline__ void load_list_counts(const int* __restrict__ cnt, in
 // sums: the tiles' entries back to back, their total, then the same in slices.
 __global__ void __launch_bounds__(kScanThreads)
 k_nb_scan_tiles(const int* __restrict__ cnt, int n, unsigned long long* __restrict__ sums,
-                int tiles, const unsigned* __restrict__ status) {
+                int tiles, const unsigned* __restrict__ ctl,
+                const unsigned* __restrict__ status) {
     __shared__ unsigned long long warp_tot[kScanThreads / 32];
-    if (__syncthreads_or(fatal(status))) return;
+    if (__syncthreads_or(fatal(status) || __ldcg(&ctl[kCtlFailed]) == 0u)) return;
     unsigned v[kScanItems];
     unsigned long long sum, slice, total, total_sliced;
     load_list_counts(cnt, n, blockIdx.x * kScanTile + threadIdx.x * kScanItems, v, sum, slice);
@@ -491,40 +558,38 @@ k_nb_scan_tiles(const int* __restrict__ cnt, int n, unsigned long long* __restri
     }
 }
 
-// One block: exclusive scans of the tile totals in place.
-__global__ void __launch_bounds__(kScanThreads)
-k_nb_scan_sums(unsigned long long* __restrict__ sums, int tiles,
-               const unsigned* __restrict__ status) {
-    __shared__ unsigned long long warp_tot[kScanThreads / 32];
-    if (__syncthreads_or(fatal(status))) return;
-    for (int way = 0; way < 2; ++way, sums += tiles + 1) {
-        unsigned long long carry = 0;
-        for (int t0 = 0; t0 < tiles; t0 += kScanThreads) {
-            const int t = t0 + threadIdx.x;
-            const unsigned long long v = t < tiles ? sums[t] : 0ull;
-            unsigned long long total;
-            const unsigned long long ex = block_scan_u64(v, warp_tot, total);
-            if (t < tiles) sums[t] = carry + ex;
-            carry += total;
-        }
-        if (threadIdx.x == 0) sums[tiles] = carry;
-    }
-}
-
 // The offsets and the step between entries, and the capacity check.
 __global__ void __launch_bounds__(kScanThreads)
 k_nb_scan_add(const int* __restrict__ cnt, int n, size_t cap,
               const unsigned long long* __restrict__ sums, int tiles, uint32_t* __restrict__ off,
-              uint32_t* __restrict__ step, unsigned* __restrict__ status) {
+              uint32_t* __restrict__ step, unsigned* __restrict__ ctl,
+              unsigned* __restrict__ status) {
     __shared__ unsigned long long warp_tot[kScanThreads / 32];
+    const bool skip = __ldcg(&ctl[kCtlFailed]) == 0u;
     if (__syncthreads_or(fatal(status))) return;
-    const bool sliced = sums[2 * tiles + 1] <= cap;
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctl[kCtlScanned] = skip ? 0u : 1u;
+    if (__syncthreads_or(skip)) return;
+    // Every block sums the tiles: before its own and in all, each way.
+    unsigned long long before[2] = {0ull, 0ull}, all[2] = {0ull, 0ull}, start[2], total[2];
+    for (int t = threadIdx.x; t < tiles; t += kScanThreads)
+#pragma unroll
+        for (int way = 0; way < 2; ++way) {
+            const unsigned long long s = sums[way * (tiles + 1) + t];
+            all[way] += s;
+            if (t < static_cast<int>(blockIdx.x)) before[way] += s;
+        }
+#pragma unroll
+    for (int way = 0; way < 2; ++way) {
+        block_scan_u64(before[way], warp_tot, start[way]);
+        block_scan_u64(all[way], warp_tot, total[way]);
+    }
+    const bool sliced = total[1] <= cap;
     const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     unsigned v[kScanItems];
-    unsigned long long sum, slice, total;
+    unsigned long long sum, slice, tile;
     load_list_counts(cnt, n, base, v, sum, slice);
-    unsigned long long run = block_scan_u64(sliced ? slice : sum, warp_tot, total) +
-                             sums[(sliced ? tiles + 1 : 0) + blockIdx.x];
+    unsigned long long run =
+        block_scan_u64(sliced ? slice : sum, warp_tot, tile) + start[sliced ? 1 : 0];
     // A slice's first thread holds its start; the others' exclusive sums are
     // past it.
     if (sliced) run = __shfl_sync(0xffffffffu, run, threadIdx.x & 31 & ~(32 / kScanItems - 1));
@@ -537,7 +602,7 @@ k_nb_scan_add(const int* __restrict__ cnt, int n, size_t cap,
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *step = sliced ? 32u : 1u;
-        if (sums[tiles] > cap) atomicOr(status, kStatusListOverflow);
+        if (total[0] > cap) atomicOr(status, kStatusListOverflow);
     }
 }
 
@@ -772,7 +837,7 @@ k_xsph(const float4* __restrict__ x, const float4* __restrict__ v,
 // The final rebuild's walk with applyXsphViscosity fused in (velocities v are
 // the updated ones, computed before this walk), and with the velocity response
 // when no vorticity pass follows.
-template <bool B>
+template <bool B, bool ALLOC>
 __global__ void PBF_GATHER_REGS(72)
 k_search_xsph(const float4* __restrict__ xs, const float* __restrict__ sx,
               const float* __restrict__ sy, const float* __restrict__ sz,
@@ -781,16 +846,17 @@ k_search_xsph(const float4* __restrict__ xs, const float* __restrict__ sx,
               const float4* __restrict__ vin, bool resolve, unsigned* __restrict__ status) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (__any_sync(0xffffffffu, fatal(status))) return;
+    if (ALLOC ? skip_alloc(c) : skip_scanned(c)) return;
     const bool active = i < n;
     i = min(i, n - 1);
     const float4 pi = xs[i], vi = v[i];
     XsphAcc s{0.0f, 0.0f, 0.0f};
-    const int count = walk_terms<B, PosVel>(
-        c, i, active, pi, sx, sy, sz, first, nbr + nb_first(c, i), c.max_nb,
+    const int count = walk_terms<B, ALLOC, PosVel>(
+        c, i, active, pi, sx, sy, sz, first, nbr, c.max_nb,
         [&](uint32_t j) { return PosVel{__ldg(&xs[j]), __ldg(&v[j])}; },
         [&](const PosVel& a, const PosVel& b) { xsph_add2(c.k, s, pi, vi, a, b); },
         [&](const PosVel& q) { xsph_add(c.k, s, pi, vi, q); });
-    if (!active) return;
+    if (!active || count < 0) return;
     cnt[i] = count;
     if (count > c.max_nb) atomicOr(status, kStatusNeighborOverflow);
     float4 out = count > c.max_nb
@@ -1099,6 +1165,21 @@ int default_walk_lanes(size_t n, int max_nb) {
     return L;
 }
 
+// The counts and offsets of compact lists, where the walk before found no place
+// for its slices.
+static void launch_count_and_scan(const float4* xs, const float* sx, const float* sy,
+                                  const float* sz, const int* first, const StepConst& c, int n,
+                                  int* cnt, unsigned* status, cudaStream_t st) {
+    const int bs = tuned_block(c, n, kTunedSearch);
+    launch_k(c.scenes ? k_count<true> : k_count<false>, blocks_for(n, bs), bs, st, xs, sx, sy, sz,
+             first, c, n, cnt, status);
+    const int tiles = static_cast<int>(blocks_for(n, kScanTile));
+    launch_k(k_nb_scan_tiles, static_cast<unsigned>(tiles), kScanThreads, st, cnt, n, c.nb_sums,
+             tiles, c.nb_ctl, status);
+    launch_k(k_nb_scan_add, static_cast<unsigned>(tiles), kScanThreads, st, cnt, n, c.nb_cap,
+             c.nb_sums, tiles, c.nb_off, c.nb_step, c.nb_ctl, status);
+}
+
 void launch_search(const float4* xs, const float* sx, const float* sy, const float* sz,
                    const int* first, const StepConst& c, int n, uint32_t* nbr, int* cnt, float* lam,
                    unsigned* status, bool with_lambda, cudaStream_t st) {
@@ -1107,19 +1188,18 @@ void launch_search(const float4* xs, const float* sx, const float* sy, const flo
         launch_search_rows(bs, xs, sx, sy, sz, first, c, n, nbr, cnt, lam, status, with_lambda, st);
         return;
     }
-    const unsigned g = blocks_for(n, bs);
-    if (with_lambda && c.scenes)
-        launch_k_smem(k_search<true, true>, g, bs, queue_bytes(bs), st, xs, sx, sy, sz, first, c, n, nbr, cnt, lam,
-                 status);
-    else if (with_lambda)
-        launch_k_smem(k_search<true, false>, g, bs, queue_bytes(bs), st, xs, sx, sy, sz, first, c, n, nbr, cnt, lam,
-                 status);
-    else if (c.scenes)
-        launch_k_smem(k_search<false, true>, g, bs, queue_bytes(bs), st, xs, sx, sy, sz, first, c, n, nbr, cnt, lam,
-                 status);
-    else
-        launch_k_smem(k_search<false, false>, g, bs, queue_bytes(bs), st, xs, sx, sy, sz, first, c, n, nbr, cnt, lam,
-                 status);
+    auto walk = [&](auto k) {
+        launch_k_smem(k, blocks_for(n, bs), bs, queue_bytes(bs), st, xs, sx, sy, sz, first, c, n,
+                      nbr, cnt, lam, status);
+    };
+    const bool b = c.scenes != nullptr;
+    if (c.nb_off) {
+        if (with_lambda) walk(b ? k_search<true, true, true> : k_search<true, false, true>);
+        else walk(b ? k_search<false, true, true> : k_search<false, false, true>);
+        launch_count_and_scan(xs, sx, sy, sz, first, c, n, cnt, status, st);
+    }
+    if (with_lambda) walk(b ? k_search<true, true, false> : k_search<true, false, false>);
+    else walk(b ? k_search<false, true, false> : k_search<false, false, false>);
 }
 
 void launch_search_xsph(const float4* xs, const float* sx, const float* sy, const float* sz,
@@ -1132,40 +1212,21 @@ void launch_search_xsph(const float4* xs, const float* sx, const float* sy, cons
                                 status, st);
         return;
     }
-    const unsigned g = blocks_for(n, bs);
-    if (c.scenes)
-        launch_k_smem(k_search_xsph<true>, g, bs, queue_bytes(bs), st, xs, sx, sy, sz, first, c, n, nbr, cnt, v, v_out,
-                 vin, resolve, status);
-    else
-        launch_k_smem(k_search_xsph<false>, g, bs, queue_bytes(bs), st, xs, sx, sy, sz, first, c, n, nbr, cnt, v, v_out,
-                 vin, resolve, status);
-}
-
-void launch_count(const float4* xs, const float* sx, const float* sy, const float* sz,
-                  const int* first, const StepConst& c, int n, int* cnt, unsigned* status,
-                  cudaStream_t st) {
-    const int bs = tuned_block(c, n, kTunedSearch);
-    const unsigned g = blocks_for(n, bs);
-    if (c.scenes)
-        launch_k(k_count<true>, g, bs, st, xs, sx, sy, sz, first, c, n, cnt, status);
-    else
-        launch_k(k_count<false>, g, bs, st, xs, sx, sy, sz, first, c, n, cnt, status);
+    auto walk = [&](auto k) {
+        launch_k_smem(k, blocks_for(n, bs), bs, queue_bytes(bs), st, xs, sx, sy, sz, first, c, n,
+                      nbr, cnt, v, v_out, vin, resolve, status);
+    };
+    const bool b = c.scenes != nullptr;
+    if (c.nb_off) {
+        walk(b ? k_search_xsph<true, true> : k_search_xsph<false, true>);
+        launch_count_and_scan(xs, sx, sy, sz, first, c, n, cnt, status, st);
+    }
+    walk(b ? k_search_xsph<true, false> : k_search_xsph<false, false>);
 }
 
 size_t nb_scan_scratch_words(size_t n) {
     const size_t tiles = (n + kScanTile - 1) / kScanTile;
     return 4 * (tiles + 1);  // 64-bit tile sums and totals, back to back and in slices
-}
-
-void launch_nb_scan(const int* cnt, uint32_t* off, uint32_t* step, size_t cap, int n,
-                    uint32_t* scratch, unsigned* status, cudaStream_t st) {
-    const int tiles = std::max(1, static_cast<int>(blocks_for(static_cast<size_t>(n), kScanTile)));
-    auto* sums = reinterpret_cast<unsigned long long*>(scratch);
-    launch_k(k_nb_scan_tiles, static_cast<unsigned>(tiles), kScanThreads, st, cnt, n, sums, tiles,
-             status);
-    launch_k(k_nb_scan_sums, 1u, kScanThreads, st, sums, tiles, status);
-    launch_k(k_nb_scan_add, static_cast<unsigned>(tiles), kScanThreads, st, cnt, n, cap, sums,
-             tiles, off, step, status);
 }
 
 template <bool B>

@@ -42,9 +42,15 @@ struct StepConst {
     // Compact neighbour lists: particle i's list is nbr[nb_off[i] + k *
     // nb_step[0]] inside nb_cap entries.  Null: slot-major lists,
     // nbr[k * stride + i].
-    const uint32_t* nb_off;
-    const uint32_t* nb_step;
+    // The walks set both; nb_ctl: kNbCtlWords words of their state, zero before
+    // a run; nb_sums: scratch of nb_scan_scratch_words(n) words; nb_retry: try
+    // slices again even if the rebuild before had no place for them.
+    uint32_t* nb_off;
+    uint32_t* nb_step;
     size_t nb_cap;
+    unsigned* nb_ctl;
+    unsigned long long* nb_sums;
+    bool nb_retry;
     // Lanes per particle in the neighbour kernels (1, 2, 4, 8, 16 or 32; 0 =
     // 1): more than one shares each particle's work over a lane group
     // (pbf_group.cu), for scenes too small to fill the GPU.  Slot-major lists
@@ -56,6 +62,8 @@ struct StepConst {
     // are; off for the stage entry points, which take the caller's tables.
     bool prune_cells;
 };
+
+constexpr size_t kNbCtlWords = 4;
 
 // Lanes per particle for the neighbour kernels of an n-particle scene
 // (slot-major lists with max_nb slots).
@@ -151,16 +159,7 @@ void launch_delta_apply(const float4* xs, const uint32_t* nbr, const int* cnt, c
                         const CellBins& bins, unsigned* status, cudaStream_t st,
                         uint8_t* moved = nullptr,
                         float4* pre = nullptr);
-// Compact lists: neighbour counts of the walk (no list written), then the
-// exclusive scan of the counts into the lists' offsets off (n entries) and
-// the step between their entries (a total above cap sets
-// kStatusListOverflow).  scratch: nb_scan_scratch_words(n) words.
-void launch_count(const float4* xs, const float* sx, const float* sy, const float* sz,
-                  const int* first, const StepConst& c, int n, int* cnt, unsigned* status,
-                  cudaStream_t st);
-size_t nb_scan_scratch_words(size_t n);
-void launch_nb_scan(const int* cnt, uint32_t* off, uint32_t* step, size_t cap, int n,
-                    uint32_t* scratch, unsigned* status, cudaStream_t st);
+size_t nb_scan_scratch_words(size_t n);  // of StepConst::nb_sums
 // The neighbour kernels of small scenes (pbf_group.cu), bs threads per block:
 // the walks with a lane per stencil row, the others with L lanes per
 // particle.  The launchers here choose them by StepConst::walk_lanes.

@@ -202,12 +202,12 @@ struct pbf_solver {
     int tuned_lanes = 0;  // lanes per particle of the walks set by pbf_set_walk_lanes; 0 = default
     int sort_tile = 0;    // keys per radix-sort tile chosen by the autotuner; 0 = by size
 
-    // Compact neighbour lists (list_cap > 0): every rebuild counts the
-    // neighbours, scans the counts into nb_off (the last word: the step
-    // between entries) and writes the lists into list_cap entries in all.
+    // Compact neighbour lists (list_cap > 0): every rebuild's walk finds the
+    // lists' places (nb_off, the last word: the step between entries) within
+    // list_cap entries in all; nb_ctl: its state.
     // 0: slot-major lists of max_nb slots per particle.
     size_t list_cap = 0;
-    DeviceBuffer nb_off, nb_scratch;
+    DeviceBuffer nb_off, nb_ctl, nb_scratch;
 
     // Device state.
     DeviceBuffer f4[kF4Pool];
@@ -311,6 +311,8 @@ struct pbf_solver {
             c.nb_off = nb_off.as<uint32_t>();
             c.nb_step = nb_off.as<uint32_t>() + cap;
             c.nb_cap = list_cap;
+            c.nb_ctl = nb_ctl.as<unsigned>();
+            c.nb_sums = nb_scratch.as<unsigned long long>();
         }
         c.walk_lanes = walk_lanes();
         c.prune_cells = true;
@@ -348,6 +350,8 @@ struct pbf_solver {
             cuda_check(cudaMemsetAsync(status.get(), 0, sizeof(unsigned), stream));
             if (bin_count.get())
                 cuda_check(cudaMemsetAsync(bin_count.get(), 0, bin_count.bytes(), stream));
+            if (nb_ctl.get())
+                cuda_check(cudaMemsetAsync(nb_ctl.get(), 0, nb_ctl.bytes(), stream));
         }
         state_dirty = true;  // until check_status
     }
@@ -358,7 +362,8 @@ struct pbf_solver {
     // the mapping from input to output roles is fixed and the captured graph
     // for a given input assignment is reusable.
     std::tuple<int, int, int> enqueue_frame(cudaStream_t st, int rx, int rv, int rid) {
-        const StepConst c = make_const();
+        StepConst c = make_const();
+        c.nb_retry = true;  // the frame's first rebuild
         const int N = static_cast<int>(n);
         unsigned* sp = status.as<unsigned>();
         bool used[kF4Pool] = {};
@@ -417,24 +422,13 @@ struct pbf_solver {
                 cur = nxt;
                 org_cur = org_next;
             };
-            // Compact lists: neighbour counts and their scan before each walk
-            // that writes lists.
-            auto count_and_scan = [&](int xs) {
-                if (list_cap == 0) return;
-                launch_count(P(xs), soa.as<float>(), soa.as<float>() + soa_stride(),
-                             soa.as<float>() + 2 * soa_stride(), cell_first.as<int>(), c, N,
-                             cnt.as<int>(), sp, st);
-                launch_nb_scan(cnt.as<int>(), nb_off.as<uint32_t>(),
-                               nb_off.as<uint32_t>() + cap, list_cap, N,
-                               nb_scratch.as<uint32_t>(), sp, st);
-            };
             for (int it = 0; it < prm.solverIterations; ++it) {
                 rebuild();
                 M(kStSearchLambda);
-                count_and_scan(cur);
                 launch_search(P(cur), soa.as<float>(), soa.as<float>() + soa_stride(),
                               soa.as<float>() + 2 * soa_stride(), cell_first.as<int>(), c, N,
                               nbr.as<uint32_t>(), cnt.as<int>(), lam.as<float>(), sp, true, st);
+                c.nb_retry = false;
                 const int nxt = take();
                 M(kStDeltaApply);
                 // Without the final rebuild nothing uses the last keys.
@@ -468,7 +462,6 @@ struct pbf_solver {
             if (xsph) {
                 const int t = take();
                 M(kStSearch);
-                count_and_scan(rx);
                 launch_search_xsph(P(rx), soa.as<float>(), soa.as<float>() + soa_stride(),
                                    soa.as<float>() + 2 * soa_stride(), cell_first.as<int>(), c,
                                    N, nbr.as<uint32_t>(), cnt.as<int>(), P(rv), P(t), P(vin2),
@@ -477,7 +470,6 @@ struct pbf_solver {
                 rv = t;
             } else if (vort) {
                 M(kStSearch);
-                count_and_scan(rx);
                 launch_search(P(rx), soa.as<float>(), soa.as<float>() + soa_stride(),
                               soa.as<float>() + 2 * soa_stride(), cell_first.as<int>(), c, N,
                               nbr.as<uint32_t>(), cnt.as<int>(), nullptr, sp, false, st);
@@ -764,9 +756,10 @@ struct pbf_solver {
         DeviceBuffer nfirst((ncells + 1) * sizeof(int));
         DeviceBuffer nsoa(3 * soa_stride_for(max_particles) * sizeof(float));
         DeviceBuffer nnbr((lcap > 0 ? lcap : strd * size_t(maxnb)) * sizeof(uint32_t));
-        DeviceBuffer nnboff, nnbscr;
+        DeviceBuffer nnboff, nnbctl, nnbscr;
         if (lcap > 0) {
             nnboff.allocate((max_particles + 1) * sizeof(uint32_t));
+            nnbctl.allocate(kNbCtlWords * sizeof(unsigned));
             nnbscr.allocate(nb_scan_scratch_words(max_particles) * sizeof(uint32_t));
         }
         DeviceBuffer ncnt(u4b), nlam(u4b);
@@ -790,6 +783,7 @@ struct pbf_solver {
         soa = std::move(nsoa);
         nbr = std::move(nnbr);
         nb_off = std::move(nnboff);
+        nb_ctl = std::move(nnbctl);
         nb_scratch = std::move(nnbscr);
         list_cap = lcap;
         cnt = std::move(ncnt);
