@@ -193,11 +193,10 @@ __device__ __forceinline__ void lambda_add2(const KernelConst& k, LambdaAcc& a, 
 // Bits of a 32-candidate chunk from j0 (the highest: candidate j0) that belong
 // to the row range [s, e), less the particle i itself.
 __device__ __forceinline__ uint32_t chunk_valid(int j0, int s, int e, int i) {
-    const int left = e - j0;
-    uint32_t valid = left >= 32 ? 0xffffffffu : ~(0xffffffffu >> left);
-    if (j0 < s) valid &= 0xffffffffu >> (s - j0);
-    const int self = i - j0;
-    if (self >= 0 && self < 32) valid &= ~(0x80000000u >> self);
+    // Shifts clamp at 32: all or nothing past the chunk's ends.
+    const uint32_t past = __funnelshift_rc(0xffffffffu, 0u, e - j0);
+    const uint32_t self = __funnelshift_rc(0x80000000u, 0u, static_cast<uint32_t>(i - j0));
+    const uint32_t valid = (0xffffffffu >> max(s - j0, 0)) & ~(past | self);
     return valid;
 }
 
@@ -372,6 +371,7 @@ __device__ __forceinline__ int walk_terms(const StepConst& c, int i, bool active
     const size_t stride = ALLOC ? 32 : nb_step(c);
     bool placed = !ALLOC;  // out is known
     bool over = false;     // hits left out of the queue
+    int steps = 0;         // chunks since the queue was empty
     int count = 0;         // neighbours handed over
     int found = 0;         // neighbours in the queue
     uint2* tail = queue;
@@ -379,6 +379,7 @@ __device__ __forceinline__ int walk_terms(const StepConst& c, int i, bool active
     auto drain = [&]() {
         const uint2* head = queue;
         uint32_t bits = 0u, j0 = 0u;
+        uint32_t* at = out + static_cast<size_t>(count) * stride;
         auto pop = [&]() {
             if (!bits) {
                 const uint2 q = *head;
@@ -386,35 +387,37 @@ __device__ __forceinline__ int walk_terms(const StepConst& c, int i, bool active
                 j0 = q.x;
                 bits = q.y;
             }
-            const int b = __clz(bits);
-            bits &= ~(0x80000000u >> b);
-            const uint32_t j = j0 + b;
-            if (count < cap) out[static_cast<size_t>(count) * stride] = j;
-            ++count;
+            const int b = 31 - __clz(bits);
+            bits ^= 1u << b;
+            const uint32_t j = j0 - b;
+            *at = j;
+            at += stride;
             return j;
         };
-        const int end = count + found;
-        while (count + 2 <= end) {
+        int left = min(found, cap - count);
+        for (; left >= 2; left -= 2) {
             const T a = load(pop()), b = load(pop());
             use2(a, b);
         }
-        if (count < end) use1(load(pop()));
+        if (left > 0) use1(load(pop()));
+        count += found;
         tail = queue;
         found = 0;
+        steps = 0;
     };
 #pragma unroll 1
     for (;;) {
         for_each_chunk<B>(c, i, active, pi, sx, sy, sz, first, [&](int j0, uint32_t bits) {
             if (bits) {
                 if (!ALLOC || tail != end_of_queue) {
-                    *tail = make_uint2(static_cast<uint32_t>(j0), bits);
+                    *tail = make_uint2(static_cast<uint32_t>(j0) + 31u, bits);
                     tail += step;
                 } else {
                     over = true;
                 }
                 found += __popc(bits);
             }
-            if (placed && __any_sync(0xffffffffu, tail == end_of_queue)) drain();
+            if (placed && (ALLOC || ++steps >= kQueue) && __any_sync(0xffffffffu, tail == end_of_queue)) drain();
         });
         if (placed) break;
         const size_t at = alloc_lists(c, min(found, cap));
