@@ -762,12 +762,7 @@ k_finalize(const uint32_t* __restrict__ org, const float4* __restrict__ x_old,
     const uint32_t o = org[i];
     const float4 xo = x_old[o];
     const float4 q = xs[i];
-    float4 vv;
-    vv.x = fmul(fsub(q.x, xo.x), c.inv_dt);
-    vv.y = fmul(fsub(q.y, xo.y), c.inv_dt);
-    vv.z = fmul(fsub(q.z, xo.z), c.inv_dt);
-    vv.w = v_old[o].w;
-    v_new[i] = vv;
+    v_new[i] = updated_velocity(xo, q, v_old[o].w, c.inv_dt);
     vin_new[i] = vin_old[o];
     if (id_new) id_new[i] = id_old[o];
 }

@@ -228,12 +228,22 @@ size_t bin_count_words(uint64_t cells);  // of CellBins::count, zeroed once
 // the particle numbers cell by cell, in arrival order.
 void launch_bin_order(const CellBins& b, const uint32_t* keys, int* first, uint32_t* list, int n,
                       uint64_t cells, const unsigned* status, cudaStream_t st);
+// The velocity update that can go with a substep's last reorder, as
+// launch_finalize does it.
+struct FinalUpdate {
+    const float4 *x_old, *vin_old, *v_old;
+    const uint32_t* id_old;
+    float4 *v_new, *vin_new;
+    uint32_t* id_new;
+    float inv_dt;
+};
 // The reorder (as launch_gather_first; perm, optional: slot -> previous slot),
 // equal keys in their previous order; clears the counts.
 void launch_bin_gather(const CellBins& b, const uint32_t* list, const uint32_t* keys,
                        const int* first, uint64_t cells, const float4* xs_in, float4* xs_out,
                        const uint32_t* org_in, uint32_t* org_out, uint32_t* perm, float* sx,
-                       float* sy, float* sz, int n, const unsigned* status, cudaStream_t st);
+                       float* sy, float* sz, int n, const unsigned* status, cudaStream_t st,
+                       const FinalUpdate* final_update = nullptr);
 
 // The grid build alone, by the same counting sort, for n <= 262,144 positions
 // in device arrays (bins_apply(n, cells)): sorted keys and indices, cell ranges

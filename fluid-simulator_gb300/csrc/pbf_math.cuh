@@ -311,4 +311,10 @@ __device__ __forceinline__ uint32_t key_of(const GridConst& g, float4 p) {
     return cell_key(g, cx, cy, cz);
 }
 
+// The velocity of a particle that moved from xo to q (w: the payload).
+__device__ __forceinline__ float4 updated_velocity(float4 xo, float4 q, float w, float inv_dt) {
+    return make_float4(fmul(fsub(q.x, xo.x), inv_dt), fmul(fsub(q.y, xo.y), inv_dt),
+                       fmul(fsub(q.z, xo.z), inv_dt), w);
+}
+
 }  // namespace pbf

@@ -48,7 +48,7 @@ namespace {
 
 constexpr int kDefaultMaxNeighbors = 256;  // kMaxNeighbors, src/pbf/pbf_solver.cu:12
 constexpr int kStrideAlignment = 256;      // neighbour stride rounding, :36-39
-constexpr int kF4Pool = 6;                 // float4 buffers rotated through roles
+constexpr int kF4Pool = 7;                 // float4 buffers rotated through roles
 
 // Stages of one frame, for the event profiler (pbf_profile_frame).
 enum Stage {
@@ -392,7 +392,7 @@ struct pbf_solver {
             launch_predict(P(rx), P(rv), P(xs0), P(vin), keys.as<uint32_t>(), bins, N, c, sp, st);
             int cur = xs0;
             int org_cur = -1;
-            auto rebuild = [&]() {
+            auto rebuild = [&](const FinalUpdate* update = nullptr) {
                 M(kStSort);
                 if (bins.count)
                     launch_bin_order(bins, keys.as<uint32_t>(), cell_first.as<int>(),
@@ -410,7 +410,7 @@ struct pbf_solver {
                                       org_cur < 0 ? nullptr : org[org_cur].as<uint32_t>(),
                                       org[org_next].as<uint32_t>(), nullptr, soa.as<float>(),
                                       soa.as<float>() + soa_stride(),
-                                      soa.as<float>() + 2 * soa_stride(), N, sp, st);
+                                      soa.as<float>() + 2 * soa_stride(), N, sp, st, update);
                 else
                     launch_gather_first(sidx.as<uint32_t>(), P(cur), P(nxt),
                                         org_cur < 0 ? nullptr : org[org_cur].as<uint32_t>(),
@@ -442,14 +442,20 @@ struct pbf_solver {
             // The final rebuild, then the velocity update (it needs only the
             // composed permutation), then the final walk: with XSPH on, the
             // walk applies XSPH in a second pass over its new lists.
-            if (post) rebuild();
             const int vnew = take();
             const int vinnew = take();
             const int idnew = 1 - rid;
+            const bool fused = post && bins.count;
+            if (post) {
+                const FinalUpdate update{P(rx), P(vin), P(rv), ids[rid].as<uint32_t>(), P(vnew),
+                                         P(vinnew), ids[idnew].as<uint32_t>(), c.inv_dt};
+                rebuild(fused ? &update : nullptr);
+            }
             M(kStFinalize);
-            launch_finalize(org[org_cur].as<uint32_t>(), P(rx), P(vin), P(rv),
-                            ids[rid].as<uint32_t>(), P(cur), N, c, P(vnew), P(vinnew),
-                            ids[idnew].as<uint32_t>(), sp, st);
+            if (!fused)
+                launch_finalize(org[org_cur].as<uint32_t>(), P(rx), P(vin), P(rv),
+                                ids[rid].as<uint32_t>(), P(cur), N, c, P(vnew), P(vinnew),
+                                ids[idnew].as<uint32_t>(), sp, st);
             give(rx);
             give(rv);
             give(vin);
