@@ -111,8 +111,9 @@ struct RowGroup {
     }
 };
 
-// Hit bits of 32 candidates of the row range [s, e) from j (a multiple of 4),
-// less the particle itself; the second 16 only as far as the range goes.
+// Hit bits of 32 candidates of the row range [s, e) from j (a multiple of 4;
+// candidate j is the highest bit), less the particle itself; 8 at a time, as
+// far as the range goes (16 at a time: 1.4 % more of a step of 16,384 particles).
 // h2u: the float above h2 (d2 <= h2 exactly when d2 - h2u has its sign set).
 __device__ __forceinline__ uint32_t row_hits(float4 pi, float h2u, const float* __restrict__ sx,
                                              const float* __restrict__ sy,
@@ -120,13 +121,13 @@ __device__ __forceinline__ uint32_t row_hits(float4 pi, float h2u, const float* 
                                              int self) {
     uint32_t acc = 0u;
 #pragma unroll 1
-    for (int t = j; t < j + 32; t += 16) {
+    for (int t = j; t < j + 32; t += 8) {
         if (t >= e) {
-            acc <<= 16;
+            acc <<= j + 32 - t;
             break;
         }
 #pragma unroll
-        for (int q = 0; q < 16; q += 4) {
+        for (int q = 0; q < 8; q += 4) {
             const float4 X = __ldg(reinterpret_cast<const float4*>(sx + t + q));
             const float4 Y = __ldg(reinterpret_cast<const float4*>(sy + t + q));
             const float4 Z = __ldg(reinterpret_cast<const float4*>(sz + t + q));
@@ -140,11 +141,9 @@ __device__ __forceinline__ uint32_t row_hits(float4 pi, float h2u, const float* 
                     acc, 1);
         }
     }
-    uint32_t m = __brev(acc);
-    if (e - j < 32) m &= (1u << (e - j)) - 1u;
-    if (s > j) m &= ~((1u << (s - j)) - 1u);
-    if (self >= j && self < j + 32) m &= ~(1u << (self - j));
-    return m;
+    const uint32_t past = __funnelshift_rc(0xffffffffu, 0u, e - j);
+    const uint32_t me = __funnelshift_rc(0x80000000u, 0u, static_cast<uint32_t>(self - j));
+    return acc & (0xffffffffu >> max(s - j, 0)) & ~(past | me);
 }
 
 // The walk of the warp's particles (slot-major or compact list at out, at
@@ -189,8 +188,9 @@ __device__ __forceinline__ int row_walk(const RowGroup& gr, const StepConst& c, 
         uint32_t m = j == a ? m0 : m1;
         if (j > a + 32) m = row_hits(pi, h2u, sx, sy, sz, j, s, e, gr.i);
         while (m) {
-            const int k = j + __ffs(m) - 1;
-            m &= m - 1u;
+            const int b = 31 - __clz(m);
+            m ^= 1u << b;
+            const int k = j + 31 - b;
             if (place < c.max_nb) *dst = static_cast<uint32_t>(k);
             if (place < kRowCap) gr.stash[place].x = __int_as_float(k);
             dst += stride;
