@@ -87,9 +87,9 @@ STAGE_BYTES = {
 # line names that frame.
 CAPTURES = {
     "search_lambda": {
-        16: {"dram_bytes": 60.676864e6 + 94.141632e6, "inst": 163705114.0},
-        106: {"dram_bytes": 111.414400e6 + 199.216960e6, "inst": 245673552.0},
-        150: {"dram_bytes": 95.744576e6 + 158.054208e6, "inst": 207600024.0},
+        16: {"dram_bytes": 39.5748e6 + 74.4403e6, "inst": 139438000.0},
+        106: {"dram_bytes": 51.9182e6 + 136.474e6, "inst": 185839000.0},
+        150: {"dram_bytes": 51.0444e6 + 112.405e6, "inst": 161953000.0},
     },
 }
 SMS, ISSUE_PER_SM_CLK = 152, 4

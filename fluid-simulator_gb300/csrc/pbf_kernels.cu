@@ -15,6 +15,7 @@
 //                                                                  collision_system.cu:133-172)
 // After the last iteration (pbf_solver.cu:260-323), after the final rebuild:
 //   k_finalize       gather x, v_in, ids by the composite permutation + velocity update
+//                    (part of the final rebuild's reorder in pbf_bins.cu)
 //   k_search_xsph    rebuilt lists for the velocity terms + XSPH over them
 //                    (k_search<false> when XSPH is off)
 //   k_vorticity, k_confine   (pbf_solver_kernels.cu:268-385), collision velocity
@@ -342,16 +343,18 @@ inline size_t queue_bytes(int threads) { return sizeof(uint2) * kQueue * threads
 // their lengths, in the first walk when the queues held all hits, else before a
 // second; -1 if there is no place left.
 //
-// Bound by instruction issue.  Appending the hits of each chunk at once costs a
-// warp the largest number of hits of any lane, chunk by chunk (2 to 3 times the
-// average), and the terms need a second pass over the list.  So the chunks with
-// hits are queued, and the lanes take their neighbours from their queues one by
-// one, in step: list entry and terms in one loop whose length is the largest
-// neighbour count.  The queues are emptied together when any is full (lanes that
-// empty theirs by themselves: walk 30 to 80 % longer in dense scenes).  Walk and
-// lambda, before and after: 38 -> 29 us at 65,536 particles, 76 -> 63 at
-// 262,144, 280 -> 222 at 1,048,576 and 875 -> 720 for 256 batched scenes; the
-// final walk with XSPH at 1,048,576 310 -> 254 (72 registers; 64 spill: 281).
+// Bound by issue (67 % active, FP32x2 operations taking two slots) and the L1's
+// data pipe (77 %: 12 bytes a lane for each candidate).  Appending the hits of
+// each chunk at once costs a warp the largest number of hits of any lane, chunk
+// by chunk (2 to 3 times the average), and the terms need a second pass over the
+// list.  So the chunks with hits are queued, and the lanes take their neighbours
+// from their queues one by one, in step: list entry and terms in one loop whose
+// length is the largest neighbour count.  The queues are emptied together when
+// any is full (lanes that empty theirs by themselves: walk 30 to 80 % longer in
+// dense scenes).  Walk and lambda, before and with all of this: 38 -> 28 us at
+// 65,536 particles, 76 -> 58 at 262,144, 280 -> 206 at 1,048,576 and 875 -> 688
+// for 256 batched scenes; the final walk with XSPH at 1,048,576 310 -> 248 (72
+// registers; 64 spill: +3 %).
 template <bool B, bool ALLOC, class T, class Load, class Use2, class Use1>
 __device__ __forceinline__ int walk_terms(const StepConst& c, int i, bool active, float4 pi,
                                           const float* __restrict__ sx,

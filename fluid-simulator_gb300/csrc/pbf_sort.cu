@@ -1,4 +1,6 @@
-// pbf_sort.cu -- stable LSD radix sort of (cell key, index) pairs.
+// pbf_sort.cu -- stable LSD radix sort of (cell key, index) pairs: the grid
+// build entry points, and the step's rebuilds where the cells are far more than
+// the particles (elsewhere pbf_bins.cu counts).
 //
 // Replaces cub::DeviceRadixSort::SortPairs over all 32 key bits
 // (src/pbf/spatial_grid.cu:188-196).  A stable sort has one result whatever

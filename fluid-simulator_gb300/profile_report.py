@@ -247,8 +247,9 @@ def main():
     kpf = int(out.split("kernels_per_frame")[1].split()[0])
     tmp_tl = tempfile.mkdtemp(prefix="pbf_tl_")
     tl_lines = timeline(args, me, shown, tmp_tl)
-    # Solver: skip set_particles (two kernels) and the warm-up frames, list
-    # one frame.  Adjoint: list every launch of the forward and backward.
+    # Solver: skip set_particles (one kernel) and the warm-up frames with their
+    # status report (one), list one frame.  Adjoint: list every launch of the
+    # forward and backward.
     before = 0 if args.adjoint else 2 + args.warmup * kpf
     tmp = tempfile.mkdtemp(prefix="pbf_prof_")
     lst = os.path.join(tmp, "launches.csv")

@@ -85,10 +85,11 @@ pbf_status pbf_initialize_ex(pbf_solver* s, size_t max_particles, pbf_float3 min
                              pbf_float3 max_bounds, const pbf_params* params,
                              int max_neighbors);
 
-/* Same with compact neighbour lists: each rebuild counts every particle's
- * neighbours, scans the counts and stores each list contiguously, list_capacity
- * entries in all (memory follows the actual neighbour count instead of
- * max_particles x max_neighbors).  Results equal those of the slot-major lists
+/* Same with compact neighbour lists: the lists of 32 consecutive particles share
+ * a slice as wide as the longest of them, or stand back to back where slices
+ * would not fit, list_capacity entries in all (memory follows the actual
+ * neighbour count instead of max_particles x max_neighbors).  A capacity of 1.3
+ * to 1.5 times the neighbours present keeps the faster slices.  Results equal those of the slot-major lists
  * bit for bit.  A step whose lists need more than list_capacity entries fails
  * with PBF_ERR_OVERFLOW; max_neighbors still bounds each particle's count as in
  * the reference.  list_capacity must be in [1, 2^32 - 1]. */
@@ -167,7 +168,8 @@ pbf_status pbf_autotune(pbf_solver* s, int frames_per_trial);
 /* The block sizes in use, in the order above (count <= 6 entries). */
 pbf_status pbf_block_sizes(const pbf_solver* s, int* sizes, int count);
 /* Keys per radix-sort tile in use: 1,024 or 4,096 (chosen by the autotuner,
- * else 1,024 below 2^19 particles and 4,096 from there on). */
+ * else 1,024 below 2^19 particles and 4,096 from there on).  Of effect only in
+ * grids of many more cells than particles: elsewhere rebuilds count. */
 pbf_status pbf_sort_tile(const pbf_solver* s, int* keys_per_tile);
 /* Lanes per particle of the list-writing walks in use: the value set by
  * pbf_set_walk_lanes, else 8 (also where small scenes take more) up to 18,432
