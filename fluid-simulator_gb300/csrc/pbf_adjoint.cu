@@ -736,12 +736,9 @@ struct pbf_adjoint {
     // arrival places, aidx the cells' lists.
     DeviceBuffer bin_count;
     CellBins cell_bins() const {
-        CellBins b;
-        if (bin_count.get()) {
-            b.count = bin_count.as<uint32_t>();
-            b.place = akeys.as<uint32_t>();
-        }
-        return b;
+        return bin_count.get()
+                   ? make_bins(bin_count.as<uint32_t>(), akeys.as<uint32_t>(), cells, n)
+                   : CellBins{};
     }
     // Tape of one segment (`every` step slots), see the accessors below.
     DeviceBuffer tf4, tu32, tlam, tnb, tcn, tmv;
@@ -994,9 +991,10 @@ struct pbf_adjoint {
         unsigned* sp = status.as<unsigned>();
         float* s0 = soa.as<float>();
         if (bin_count.get()) {
-            launch_bin_order(cell_bins(), keys.as<uint32_t>(), first.as<int>(), aidx.as<uint32_t>(),
+            const CellBins bins = cell_bins();
+            launch_bin_order(org_in ? bins : bins.without_sums(), keys.as<uint32_t>(), first.as<int>(), aidx.as<uint32_t>(),
                              N, cells, sp, stream);
-            launch_bin_gather(cell_bins(), aidx.as<uint32_t>(), keys.as<uint32_t>(),
+            launch_bin_gather(bins, aidx.as<uint32_t>(), keys.as<uint32_t>(),
                               first.as<int>(), cells, src, dst, org_in, org_out, rel, s0,
                               s0 + soa_stride(), s0 + 2 * soa_stride(), N, sp, stream);
             return;

@@ -20,12 +20,12 @@
 // at least as many pairs of each cell, so no distribution of the particles
 // makes it the larger cost.
 //
-// Bound by the latency of its dependent loads and, up to some 100,000
-// particles, by its launches (2 a rebuild up to 8,192 cells, 3 to 32,768, 4
-// above) against the radix sort's 4 to 9 small ones and the gather's search of
+// Bound by the latency of its dependent loads (2 launches a rebuild up to 8,192
+// cells, 3 above, and one more where the scan's tile sums are not counted with
+// the keys) against the radix sort's 4 to 9 launches and the gather's search of
 // first[].  Measured on a GB300, radix sort and gather against this, five
-// rebuilds of a frame: 81 -> 64 us at 1,024 particles, 137 -> 93 at 65,536,
-// 387 -> 241 at 262,144 (two substeps), 310 -> 196 at 1,048,576, 1.67 -> 1.07
+// rebuilds of a frame: 81 -> 64 us at 1,024 particles, 137 -> 85 at 65,536,
+// 387 -> 215 at 262,144 (two substeps), 310 -> 196 at 1,048,576, 1.67 -> 1.07
 // ms at 8,388,608.
 #include "pbf_kernels.cuh"
 
@@ -125,12 +125,28 @@ k_bin_small(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ plac
 }
 
 constexpr int kScanThreads = 512;
-// Up to kDirectCells the scan's blocks sum the counts before their own tile
-// themselves; above, the tiles' sums come from a launch of their own (in the
-// words after the counts; at 32,768 cells 3.8 + 5.9 us against 5.4).  Tiles of
-// kFew cells a thread up to kFewCells (32,768 cells: 8.4 -> 5.4 us).
+// A scan block's tile of counts: kFew cells a thread up to kFewCells (32,768
+// cells: 8.4 -> 5.4 us), kMany above.  The tiles' sums are counted with the keys
+// (put_key), a warp's particles of a tile at once, where the particles are in the
+// last rebuild's order and at most kTileCountMax: frame at 65,536 particles 244 ->
+// 238 us, pass at 262,144 (two substeps) 2,174 -> 2,150; at 8,388,608 the atomics
+// cost more than they save (13.6 -> 14.2 ms), and with particles in any order
+// neighbouring threads share no tile (200,003 positions 31 -> 70 us).  Else
+// k_bin_sums reads the counts (5.0 us at 1,048,576 particles) or, up to
+// kDirectCells, every scan block those before its own tile (at 32,768 cells 5.4 us
+// against 3.8 + 5.9).
 constexpr uint32_t kDirectCells = 32768;
+constexpr size_t kTileCountMax = size_t(1) << 19;
 constexpr uint32_t kFewCells = 1u << 20;
+int tile_shift(uint64_t cells) {
+    constexpr int few = 10, many = 12;
+    static_assert(kScanThreads * kFew == 1 << few && kScanThreads * kMany == 1 << many, "");
+    return cells <= kFewCells ? few : many;
+}
+size_t tile_count(uint64_t cells) {
+    return static_cast<size_t>((cells + (uint64_t(1) << tile_shift(cells)) - 1) >>
+                               tile_shift(cells));
+}
 
 template <int ITEMS, bool PADDED = true>
 __global__ void __launch_bounds__(kScanThreads)
@@ -189,20 +205,21 @@ k_bin_scatter(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ pl
 }
 
 // Thread s < n reorders the particle in slot s; thread s < cells clears the
-// count of cell s for the next rebuild.  FINAL: with the velocity update of
+// count of cell s (s < tiles: the sum of tile s) for the next rebuild.  FINAL: with the velocity update of
 // k_finalize for the same particle (as a launch of its own it adds 2 us to a
 // frame of up to 65,536 particles, 11 to one of 1,048,576).
 template <bool FINAL>
 __global__ void __launch_bounds__(kBlock)
 k_bin_gather(const uint32_t* __restrict__ list, const uint32_t* __restrict__ keys,
              const int* __restrict__ first, uint32_t* __restrict__ count, uint32_t cells,
-             const float4* __restrict__ xs_in, float4* __restrict__ xs_out,
+             uint32_t* __restrict__ sums, uint32_t tiles, const float4* __restrict__ xs_in, float4* __restrict__ xs_out,
              const uint32_t* __restrict__ org_in, uint32_t* __restrict__ org_out,
              uint32_t* __restrict__ perm, float* __restrict__ sx, float* __restrict__ sy,
              float* __restrict__ sz, int n, FinalUpdate f, const unsigned* __restrict__ status) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (fatal(status)) return;
     if (static_cast<uint32_t>(s) < cells) count[s] = 0u;
+    if (static_cast<uint32_t>(s) < tiles) sums[s] = 0u;
     if (s >= n) return;
     const uint32_t p = list[s];
     const uint32_t key = keys[p];
@@ -391,8 +408,23 @@ bool bins_apply(size_t n, uint64_t cells) {
 }
 
 size_t bin_count_words(uint64_t cells) {
-    const uint64_t tile = kScanThreads * (cells <= kFewCells ? kFew : kMany);
-    return static_cast<size_t>((cells + kMany - 1) / kMany * kMany + (cells + tile - 1) / tile);
+    return static_cast<size_t>((cells + kMany - 1) / kMany * kMany) + tile_count(cells);
+}
+
+// Above kSmallCells cells the words after the counts hold the tiles' sums.
+static uint32_t* sums_of(const CellBins& b, uint64_t cells) {
+    return b.count + (cells + kMany - 1) / kMany * kMany;
+}
+
+CellBins make_bins(uint32_t* count, uint32_t* place, uint64_t cells, size_t n) {
+    CellBins b;
+    b.count = count;
+    b.place = place;
+    if (cells > kSmallCells && n <= kTileCountMax) {
+        b.sums = sums_of(b, cells);
+        b.shift = tile_shift(cells);
+    }
+    return b;
 }
 
 void launch_bin_order(const CellBins& b, const uint32_t* keys, int* first, uint32_t* list, int n,
@@ -404,10 +436,10 @@ void launch_bin_order(const CellBins& b, const uint32_t* keys, int* first, uint3
         return;
     }
     const bool few = nc <= kFewCells;
-    const unsigned tiles = blocks_for(nc, kScanThreads * (few ? kFew : kMany));
-    uint32_t* sums = nullptr;
-    if (nc > kDirectCells) {
-        sums = b.count + (nc + kMany - 1) / kMany * kMany;
+    const unsigned tiles = static_cast<unsigned>(tile_count(cells));
+    uint32_t* sums = b.sums;
+    if (!sums && nc > kDirectCells) {
+        sums = sums_of(b, cells);
         launch_k(few ? k_bin_sums<kFew> : k_bin_sums<kMany>, tiles, kScanThreads, st, b.count, nc,
                  sums, status);
     }
@@ -423,13 +455,13 @@ void launch_bin_gather(const CellBins& b, const uint32_t* list, const uint32_t* 
                        const FinalUpdate* final_update) {
     const uint64_t threads = std::max<uint64_t>(static_cast<uint64_t>(n), cells);
     launch_k(final_update ? k_bin_gather<true> : k_bin_gather<false>, blocks_for(threads), kBlock, st, list, keys, first, b.count,
-             static_cast<uint32_t>(cells), xs_in, xs_out, org_in, org_out, perm, sx, sy, sz, n,
+             static_cast<uint32_t>(cells), b.sums,
+             b.sums ? static_cast<uint32_t>(tile_count(cells)) : 0u, xs_in, xs_out, org_in, org_out, perm, sx, sy, sz, n,
              final_update ? *final_update : FinalUpdate{}, status);
 }
 
 size_t bin_grid_words(uint64_t cells) {
-    const uint64_t tile = kScanThreads * (cells <= kFewCells ? kFew : kMany);
-    return static_cast<size_t>((cells + tile - 1) / tile) + 1 + kUnits;
+    return tile_count(cells) + 1 + kUnits;
 }
 
 void launch_bin_grid(const float4* pos, int n, const GridConst& g, uint64_t cells,
@@ -438,7 +470,7 @@ void launch_bin_grid(const float4* pos, int n, const GridConst& g, uint64_t cell
                      cudaStream_t st) {
     const uint32_t nc = static_cast<uint32_t>(cells);
     const bool few = nc <= kFewCells;
-    const unsigned tiles = blocks_for(nc, kScanThreads * (few ? kFew : kMany));
+    const unsigned tiles = static_cast<unsigned>(tile_count(cells));
     uint32_t* count = reinterpret_cast<uint32_t*>(cell_start);
     uint32_t *sums = scratch, *units = scratch + tiles;
     launch_error_check(cudaMemsetAsync(count, 0, cells * sizeof(uint32_t), st));

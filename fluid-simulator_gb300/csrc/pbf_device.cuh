@@ -60,6 +60,7 @@ __device__ __forceinline__ void put_key(uint32_t* __restrict__ keys, const CellB
                                         uint32_t key) {
     keys[i] = key;
     if (bins.count) bins.place[i] = atomicAdd(&bins.count[key], 1u);
+    if (bins.sums) count_tile(bins.sums, bins.shift, key);
 }
 
 // Accumulated constraint terms of computeLambda (pbf_solver_kernels.cu:26-105).

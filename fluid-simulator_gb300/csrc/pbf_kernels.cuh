@@ -118,10 +118,19 @@ inline void launch_k(void (*k)(P...), unsigned grid, unsigned block, cudaStream_
 
 // Counting-sort state of one solver (pbf_bins.cu): count[cell] (zero between
 // rebuilds) and every particle's place among its cell's arrivals, written with
-// the keys.  count null: keys only.
+// the keys.  count null: keys only.  sums (optional, zero between rebuilds): the
+// sums of the scan's tiles of 2^shift cells are counted too, for particles in the
+// last rebuild's order; without_sums for others.
 struct CellBins {
     uint32_t* count = nullptr;
     uint32_t* place = nullptr;
+    uint32_t* sums = nullptr;
+    int shift = 0;
+    CellBins without_sums() const {
+        CellBins b = *this;
+        b.sums = nullptr;
+        return b;
+    }
 };
 
 // --- step kernels (pbf_kernels.cu) -----------------------------------------
@@ -224,6 +233,16 @@ void launch_integrate(const float4* x, float4* xs, float4* v, int n, const StepC
 // Whether the step's rebuilds use it: cells in proportion to the particles.
 bool bins_apply(size_t n, uint64_t cells);
 size_t bin_count_words(uint64_t cells);  // of CellBins::count, zeroed once
+CellBins make_bins(uint32_t* count, uint32_t* place, uint64_t cells, size_t n);
+#ifdef __CUDACC__
+// Adds the particle's key to its tile: one atomic a warp and tile, by the lanes
+// that are active.
+__device__ __forceinline__ void count_tile(uint32_t* __restrict__ sums, int shift, uint32_t key) {
+    const unsigned same = __match_any_sync(__activemask(), key >> shift);
+    if (static_cast<int>(threadIdx.x & 31u) == __ffs(same) - 1)
+        atomicAdd(&sums[key >> shift], static_cast<uint32_t>(__popc(same)));
+}
+#endif
 // From keys and their counts: the cell table first[] (cells + 1 entries) and
 // the particle numbers cell by cell, in arrival order.
 void launch_bin_order(const CellBins& b, const uint32_t* keys, int* first, uint32_t* list, int n,

@@ -336,12 +336,9 @@ struct pbf_solver {
 
     // The counting sort's state when the rebuilds use it.
     CellBins cell_bins() const {
-        CellBins b;
-        if (bin_count.get()) {
-            b.count = bin_count.as<uint32_t>();
-            b.place = akeys.as<uint32_t>();
-        }
-        return b;
+        return bin_count.get()
+                   ? make_bins(bin_count.as<uint32_t>(), akeys.as<uint32_t>(), cells, cap)
+                   : CellBins{};
     }
     // Before the first frame of a run: status and counts, unless the last run
     // is known to have ended well.
@@ -389,13 +386,15 @@ struct pbf_solver {
             const int xs0 = take();
             const int vin = take();
             M(kStPredict);
-            launch_predict(P(rx), P(rv), P(xs0), P(vin), keys.as<uint32_t>(), bins, N, c, sp, st);
+            launch_predict(P(rx), P(rv), P(xs0), P(vin), keys.as<uint32_t>(), bins.without_sums(),
+                           N, c, sp, st);
             int cur = xs0;
             int org_cur = -1;
             auto rebuild = [&](const FinalUpdate* update = nullptr) {
                 M(kStSort);
                 if (bins.count)
-                    launch_bin_order(bins, keys.as<uint32_t>(), cell_first.as<int>(),
+                    launch_bin_order(org_cur < 0 ? bins.without_sums() : bins,
+                                     keys.as<uint32_t>(), cell_first.as<int>(),
                                      aidx.as<uint32_t>(), N, cells, sp, st);
                 else
                     launch_sort(plan, keys.as<uint32_t>(), skeys.as<uint32_t>(),
