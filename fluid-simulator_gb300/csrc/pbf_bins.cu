@@ -74,21 +74,21 @@ template <int ITEMS, bool PADDED = true>
 __device__ __forceinline__ uint32_t load_counts(const uint32_t* __restrict__ count, uint32_t at,
                                                 uint32_t cells, uint32_t (&v)[ITEMS]) {
     uint32_t sum = 0u;
-    if constexpr (!PADDED) {
+    if constexpr (PADDED) {
+#pragma unroll
+        for (int q = 0; q < ITEMS; q += 2) {
+            const uint2 w = at + q < cells ? __ldcg(reinterpret_cast<const uint2*>(count + at + q))
+                                           : make_uint2(0u, 0u);
+            v[q] = w.x;
+            v[q + 1] = w.y;
+            sum += w.x + w.y;
+        }
+    } else {
 #pragma unroll
         for (int q = 0; q < ITEMS; ++q) {
             v[q] = at + q < cells ? __ldcg(&count[at + q]) : 0u;
             sum += v[q];
         }
-        return sum;
-    }
-#pragma unroll
-    for (int q = 0; q < ITEMS; q += 2) {
-        const uint2 w = at + q < cells ? __ldcg(reinterpret_cast<const uint2*>(count + at + q))
-                                       : make_uint2(0u, 0u);
-        v[q] = w.x;
-        v[q + 1] = w.y;
-        sum += w.x + w.y;
     }
     return sum;
 }
