@@ -214,10 +214,14 @@ struct pbf_solver {
     DeviceBuffer ids[2], org[2];
     DeviceBuffer keys, skeys, sidx, akeys, aidx;
     // Counting sort (bins): the cells' counts; akeys holds the arrival places
-    // and aidx the lists.  The counts and the status are zero between runs,
-    // except after a failed or unchecked one (state_dirty).
+    // and aidx the lists.
     DeviceBuffer bin_count;
-    bool state_dirty = true;
+    // Whether status, counts and nb_ctl are zero, as a run needs them: kClean
+    // once a run that was enqueued whole has ended well, the only way a run's
+    // kernels leave them so.  Fresh buffers, a run that failed and one that was
+    // not enqueued to its end are kDirty whatever the status reads.
+    enum RunState { kDirty, kEnqueued, kClean };
+    RunState run_state = kDirty;
     DeviceBuffer cell_first, nbr, cnt, lam, sort_scratch, status, tmp4;
     DeviceBuffer soa;  // x, y, z components of the reordered predicted positions
     // Component array stride (see soa_stride_for).
@@ -343,14 +347,14 @@ struct pbf_solver {
     // Before the first frame of a run: status and counts, unless the last run
     // is known to have ended well.
     void clear_status() {
-        if (state_dirty) {
+        if (run_state != kClean) {
             cuda_check(cudaMemsetAsync(status.get(), 0, sizeof(unsigned), stream));
             if (bin_count.get())
                 cuda_check(cudaMemsetAsync(bin_count.get(), 0, bin_count.bytes(), stream));
             if (nb_ctl.get())
                 cuda_check(cudaMemsetAsync(nb_ctl.get(), 0, nb_ctl.bytes(), stream));
         }
-        state_dirty = true;  // until check_status
+        run_state = kDirty;
     }
 
     // ---- frame emission -----------------------------------------------------
@@ -565,6 +569,7 @@ struct pbf_solver {
         auto& g = graph_for(ix, iv, iid, true);
         cuda_check(cudaGraphLaunch(g.first, stream));
         std::tie(ix, iv, iid) = g.second;
+        run_state = kEnqueued;
         check_status();
         for (int k = 0; k < kStageCount; ++k) {
             ms[k] = 0.0f;
@@ -690,7 +695,7 @@ struct pbf_solver {
         if (s & kStatusNotConverged) fail(PBF_ERR_RUNTIME, "Collision constraints did not converge");
         if (s & kStatusListOverflow)
             fail(PBF_ERR_OVERFLOW, "Neighbor lists exceed the compact list capacity");
-        state_dirty = false;
+        if (run_state == kEnqueued) run_state = kClean;
     }
 
     void run_frames(size_t frames, bool sync) {
@@ -699,6 +704,7 @@ struct pbf_solver {
         upload_colliders();
         clear_status();
         enqueue_frames(frames);
+        run_state = kEnqueued;
         if (sync) check_status();
     }
 
@@ -782,7 +788,7 @@ struct pbf_solver {
         akeys = std::move(nakeys);
         aidx = std::move(naidx);
         bin_count = std::move(nbins);
-        state_dirty = true;
+        run_state = kDirty;
         cuda_check(cudaMemsetAsync(aidx.get(), 0, u4b, stream));
         cell_first = std::move(nfirst);
         soa = std::move(nsoa);
