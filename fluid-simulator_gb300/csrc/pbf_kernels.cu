@@ -258,9 +258,15 @@ __device__ __forceinline__ void for_each_chunk(const StepConst& c, int i, bool a
         acc = __funnelshift_l(__float_as_uint(b0), acc, 1);
         acc = __funnelshift_l(__float_as_uint(b1), acc, 1);
     };
-    const int R = __reduce_max_sync(0xffffffffu, rows.g.radius);  // of the warp's scenes
-    for (int dz = -R; dz <= R; ++dz)
-        for (int dy = -R; dy <= R; ++dy) {
+    // Steps of the warp: the radius, as far as the grid has rows (a stage call's
+    // radius may reach far past a thin grid); of the warp's scenes.
+    int Rz = min(rows.g.radius, rows.g.gz - 1), Ry = min(rows.g.radius, rows.g.gy - 1);
+    if constexpr (B) {
+        Rz = __reduce_max_sync(0xffffffffu, Rz);
+        Ry = __reduce_max_sync(0xffffffffu, Ry);
+    }
+    for (int dz = -Rz; dz <= Rz; ++dz)
+        for (int dy = -Ry; dy <= Ry; ++dy) {
             const int z = rows.cz + dz, y = rows.cy + dy;
             int s = 0, e = 0;
             if (!active || z < rows.z0 || z > rows.z1 || y < rows.y0 || y > rows.y1 ||
