@@ -36,8 +36,12 @@ std::array<int, 3> grid_dims_checked(pbf_float3 mn, pbf_float3 mx, float cell);
 // boxes (center, -), (halfExtents, -), 2 planes (point, -), (normal, -).
 std::vector<float4> collider_records(int kind, const void* data, size_t count);
 
+// (Takes the error off the runtime's record, so that a call refused once does not
+// fail the next one's launch check.)
 inline void cuda_check(cudaError_t e) {
-    if (e != cudaSuccess) fail(PBF_ERR_RUNTIME, cudaGetErrorString(e));
+    if (e == cudaSuccess) return;
+    cudaGetLastError();
+    fail(PBF_ERR_RUNTIME, cudaGetErrorString(e));
 }
 
 // An NVTX range around one entry point, for a timeline tool (Nsight Systems)

@@ -17,6 +17,8 @@
 #include "pbf_common.h"
 #include "pbf_kernels.cuh"
 
+#include <cuda.h>
+
 #include <algorithm>
 #include <array>
 #include <cmath>
@@ -45,6 +47,28 @@ void set_global_error(const std::string& m) {
 using namespace pbf;
 
 namespace {
+
+// Bytes from p to the end of the device allocation that holds it; 0 if there is
+// none.
+size_t allocation_left(const void* p) {
+    using GetRange = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+    static const GetRange get = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found{};
+        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000,
+                                             cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<GetRange>(f);
+    }();
+    const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    if (!get || get(&base, &size, at) != CUDA_SUCCESS || at < base || at - base >= size) return 0;
+    return size - (at - base);
+}
 
 constexpr int kDefaultMaxNeighbors = 256;  // kMaxNeighbors, src/pbf/pbf_solver.cu:12
 constexpr int kStrideAlignment = 256;      // neighbour stride rounding, :36-39
@@ -930,7 +954,7 @@ struct pbf_solver {
             if (i != ix && i != iv) spare[k++] = i;
         const int nid = 1 - iid;
         float4 *px = f4[spare[0]].as<float4>(), *pv = f4[spare[1]].as<float4>();
-        if (device_ptrs && kernel_can_use(pos) && kernel_can_use(vel)) {
+        if (device_ptrs && kernel_can_use(pos, count) && kernel_can_use(vel, count)) {
             take_particles(pos, vel, px, pv, ids[nid].as<uint32_t>(), count);
         } else {
             const cudaMemcpyKind kind =
@@ -950,18 +974,32 @@ struct pbf_solver {
                         size_t count);
     void report_status();
 
-    // Whether a kernel may take a caller's array in place of a copy: 16-byte
-    // aligned memory of this device (or managed).  Anything else, a host
-    // address among it, goes through cudaMemcpy and its own checks.
-    bool kernel_can_use(const void* p) const {
+    // Whether a kernel may take a caller's array of count elements in place of a
+    // copy: 16-byte aligned memory of this device (or managed), inside one
+    // allocation.  Anything else, a host address among it, goes through
+    // cudaMemcpy and its own checks; an array that reaches past the end of device
+    // memory is refused here with the status that the copy gives it.
+    bool kernel_can_use(const void* p, size_t count) const {
         cudaPointerAttributes a{};
         if (reinterpret_cast<uintptr_t>(p) % sizeof(float4) != 0) return false;
         if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
             cudaGetLastError();
             return false;
         }
-        return (a.type == cudaMemoryTypeDevice && a.device == device) ||
-               a.type == cudaMemoryTypeManaged;
+        if (!((a.type == cudaMemoryTypeDevice && a.device == device) ||
+              a.type == cudaMemoryTypeManaged))
+            return false;
+        const size_t left = allocation_left(p);
+        if (left >= count * sizeof(float4)) return true;
+        if (left == 0) return false;  // not known: the copy decides
+        // Past its allocation, but in the next ones all the way: mappings side by
+        // side may hold one array, and the copy decides.
+        for (size_t at = left; at < count * sizeof(float4);) {
+            const size_t more = allocation_left(static_cast<const char*>(p) + at);
+            if (more == 0) cuda_check(cudaErrorInvalidValue);
+            at += more;
+        }
+        return false;
     }
 
     void copy_out(bool velocities, float4* out, size_t count, bool device_ptr) {
@@ -973,7 +1011,7 @@ struct pbf_solver {
         use_device();
         if (out == nullptr) fail(PBF_ERR_INVALID_ARGUMENT, "Destination cannot be null");
         // Back in API order: straight into a device array, through tmp4 else.
-        const bool direct = device_ptr && kernel_can_use(out);
+        const bool direct = device_ptr && kernel_can_use(out, count);
         launch_scatter_by_id(f4[velocities ? iv : ix].as<float4>(), ids[iid].as<uint32_t>(),
                              direct ? out : tmp4.as<float4>(), static_cast<int>(count), stream);
         cuda_check(cudaGetLastError());
