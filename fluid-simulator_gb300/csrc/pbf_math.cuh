@@ -167,16 +167,18 @@ __device__ __forceinline__ float spiky_scale(const KernelConst& k, float d2) {
     const float t = ffma(-r, k.inv_h, 1.0f);
     return fmul(fmul(k.c_spiky, fmul(t, t)), rr);
 }
-// (Zero as a scale of 0: d * 0 may be -0, which leaves every sum unchanged.)
+// (Zero whatever the difference: a caller's list may name a pair whose difference
+// is infinite, and infinity times a scale of 0 is no number.)
 __device__ __forceinline__ void spiky(const KernelConst& k, float dx, float dy, float dz,
                                       float d2, float& gx, float& gy, float& gz) {
-    const float sc = spiky_scale(k, d2);
-    const float s = d2 < kSpikyMinD2 || d2 >= k.h2 ? 0.0f : sc;
-    gx = fmul(dx, s);
-    gy = fmul(dy, s);
-    gz = fmul(dz, s);
+    const float s = spiky_scale(k, d2);
+    const bool zero = d2 < kSpikyMinD2 || d2 >= k.h2;
+    gx = zero ? 0.0f : fmul(dx, s);
+    gy = zero ? 0.0f : fmul(dy, s);
+    gz = zero ? 0.0f : fmul(dz, s);
 }
-// The scale s of two squared distances, 0 where spiky() returns zero.
+// The scale s of two squared distances, 0 where spiky() returns zero
+// (d * 0 may then be -0, which leaves every sum it enters unchanged).
 __device__ __forceinline__ f32x2 spiky_scale2(const KernelConst& k, f32x2 d2) {
     const f32x2 rr = rsqrt_nt2(d2);
     const f32x2 r = mul2(d2, rr);
