@@ -397,13 +397,13 @@ class PBFSolver:
         return dict(zip(self.TUNED_KERNELS, list(out)), sort_tile=tile.value)
 
     def walk_lanes(self) -> int:
-        """Lanes per particle of the list-writing walks (pbf_walk_lanes)."""
+        """Lanes per particle of the neighbour kernels, 8 for 8 or more (pbf_walk_lanes)."""
         k = C.c_int()
         self._check(self._L.pbf_walk_lanes(self._h, C.byref(k)))
         return k.value
 
     def set_walk_lanes(self, lanes: int):
-        """pbf_set_walk_lanes: 1, 2, 4 or 8 lanes per particle, 0 = default."""
+        """pbf_set_walk_lanes: 1, 2, 4 or 8 (or more) lanes per particle, 0 = default."""
         self._check(self._L.pbf_set_walk_lanes(self._h, int(lanes)))
 
     def set_particles(self, positions, velocities, count: Optional[int] = None):

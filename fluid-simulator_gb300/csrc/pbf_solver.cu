@@ -702,11 +702,15 @@ struct pbf_solver {
         sort_tile = best_tile;
     }
 
-    // Lanes per particle of the list-writing walks: the value set, else the
-    // default for the scene size; 1 with compact lists.
+    // Lanes per particle of the neighbour kernels: the value set, else the
+    // default for the scene size; 1 with compact lists.  8 set stands for the
+    // default's 16 or 32 too (small scenes), as pbf_walk_lanes reports them: a
+    // caller that sets what it read changes nothing.
     int walk_lanes() const {
         if (list_cap > 0) return 1;
-        const int L = tuned_lanes > 0 ? tuned_lanes : default_walk_lanes(n, max_nb);
+        const int by_size = default_walk_lanes(n, max_nb);
+        const int L = tuned_lanes == 0 || tuned_lanes == 8 ? std::max(tuned_lanes, by_size)
+                                                           : tuned_lanes;
         return max_nb >= L && n * size_t(L) <= (size_t(1) << 30) ? L : 1;
     }
 

@@ -171,13 +171,14 @@ pbf_status pbf_block_sizes(const pbf_solver* s, int* sizes, int count);
  * else 1,024 below 2^19 particles and 4,096 from there on).  Of effect only in
  * grids of many more cells than particles: elsewhere rebuilds count. */
 pbf_status pbf_sort_tile(const pbf_solver* s, int* keys_per_tile);
-/* Lanes per particle of the list-writing walks in use: the value set by
- * pbf_set_walk_lanes, else 8 (also where small scenes take more) up to 18,432
- * particles and 1 from there on (always 1 with compact lists; at most
- * max_neighbors). */
+/* Lanes per particle of the neighbour kernels: the value set by
+ * pbf_set_walk_lanes, else 8 up to 18,432 particles and 1 from there on (always 1
+ * with compact lists; at most max_neighbors).  8 stands for 8 or more: scenes of up
+ * to 10,240 particles run 16, of up to 3,072 32, by default and with 8 set. */
 pbf_status pbf_walk_lanes(const pbf_solver* s, int* lanes);
-/* Sets the lanes per particle of the walks: 1, 2, 4 or 8, or 0 for the
- * default by scene size.  Results do not change.  A lane group pays when one small
+/* Sets the lanes per particle of the neighbour kernels: 1, 2, 4, 8 (or more, as
+ * above), or 0 for the default by scene size.  Setting the value that
+ * pbf_walk_lanes gives changes nothing.  Results do not change.  A lane group pays when one small
  * scene leaves the GPU idle; many small solvers running at once on separate
  * streams fill it already and step faster with 1. */
 pbf_status pbf_set_walk_lanes(pbf_solver* s, int lanes);
