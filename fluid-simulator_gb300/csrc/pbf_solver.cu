@@ -610,8 +610,9 @@ struct pbf_solver {
     // Autotuner: for each tuned kernel, time its stage in profiled frames at
     // 64, 128, 256 and 512 threads per block and keep the fastest (coordinate
     // descent, one kernel at a time; the other kernels keep their current
-    // sizes); then the radix sort's tile (1,024 keys in 256-thread blocks or
-    // 4,096 keys in 512-thread blocks), timed on the sort stage.  Neither
+    // sizes); then, where the rebuilds sort by digits, the radix sort's tile
+    // (1,024 keys in 256-thread blocks or 4,096 keys in 512-thread blocks), timed
+    // on the sort stage.  Neither
     // changes any arithmetic or the sort's result, so results stay bit for
     // bit the same.  The particle state is saved before and restored after,
     // so tuning does not advance the simulation.
@@ -681,7 +682,9 @@ struct pbf_solver {
             }
             tuned[k] = best;
         }
-        // The sort tile, timed on the sort stage of the same frames.
+        // The sort tile, timed on the sort stage of the same frames; nothing to
+        // time where the rebuilds count.
+        if (bin_count.get()) return;
         int best_tile = sort_tile;
         float best_ms = -1.0f;
         for (int tile : {kSortMinTile, kSortMaxTile}) {

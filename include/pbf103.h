@@ -160,8 +160,8 @@ int pbf_batch_scene_count(const pbf_solver* s);
  * kernels (walk + lambda, delta p, final walk, XSPH, vorticity,
  * confinement), times each at 64, 128, 256 and 512 threads per block in profiled
  * frames (`frames_per_trial` per size, after two untimed frames) and keeps
- * the fastest; then the radix sort's tile, 1,024 or 4,096 keys, timed on the
- * sort stage.  Results do not change (neither changes any arithmetic or the
+ * the fastest; then, in grids where the rebuilds sort by digits (pbf_sort_tile),
+ * the radix sort's tile, 1,024 or 4,096 keys, timed on the sort stage.  Results do not change (neither changes any arithmetic or the
  * sort's result); the particle state is restored, so tuning does not advance
  * the simulation.  Needs particles set. */
 pbf_status pbf_autotune(pbf_solver* s, int frames_per_trial);
