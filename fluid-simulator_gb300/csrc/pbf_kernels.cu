@@ -1109,7 +1109,7 @@ void launch_predict(const float4* x, const float4* v, float4* xs, float4* vin, u
                     const CellBins& bins, int n, const StepConst& c, const unsigned* status,
                     cudaStream_t st) {
     launch_k(c.scenes ? k_predict<true> : k_predict<false>, blocks_for(n), kBlock, st, x, v, xs,
-             vin, keys, bins, n, c, status);
+             vin, keys, bins.without_sums(), n, c, status);
 }
 void launch_cell_ranges(const uint32_t* skeys, int* cs, int* ce, int n, const unsigned* status,
                         cudaStream_t st) {

@@ -134,6 +134,9 @@ struct CellBins {
 };
 
 // --- step kernels (pbf_kernels.cu) -----------------------------------------
+// Keys are counted without the tiles' sums: the particles are not in the last
+// rebuild's order (a step taped in the order of ids), and the first rebuild after
+// it takes without_sums().
 void launch_predict(const float4* x, const float4* v, float4* xs, float4* vin, uint32_t* keys,
                     const CellBins& bins, int n, const StepConst& c, const unsigned* status,
                     cudaStream_t st);

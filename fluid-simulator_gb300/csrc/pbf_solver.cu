@@ -414,8 +414,7 @@ struct pbf_solver {
             const int xs0 = take();
             const int vin = take();
             M(kStPredict);
-            launch_predict(P(rx), P(rv), P(xs0), P(vin), keys.as<uint32_t>(), bins.without_sums(),
-                           N, c, sp, st);
+            launch_predict(P(rx), P(rv), P(xs0), P(vin), keys.as<uint32_t>(), bins, N, c, sp, st);
             int cur = xs0;
             int org_cur = -1;
             auto rebuild = [&](const FinalUpdate* update = nullptr) {
