@@ -892,17 +892,19 @@ struct pbf_adjoint {
         const size_t f4b = n * sizeof(float4), u4b = n * sizeof(uint32_t);
         const size_t E = static_cast<size_t>(every), I = static_cast<size_t>(iters);
         keys.allocate(u4b);
-        skeys.allocate(u4b);
         akeys.allocate(u4b);
         aidx.allocate(u4b);
         orgs.allocate(2 * u4b);
         first.allocate((cells + 1) * sizeof(int));
-        if (bins_apply(n, cells))
+        // The rebuilds' counting sort, or the radix sort's buffers.
+        for (DeviceBuffer* b : {&bin_count, &skeys, &scratch}) *b = DeviceBuffer();
+        if (bins_apply(n, cells)) {
             bin_count.allocate(bin_count_words(cells) * sizeof(uint32_t));
-        else
-            bin_count = DeviceBuffer();
+        } else {
+            skeys.allocate(u4b);
+            scratch.allocate(sort_scratch_bytes(static_cast<int>(n)));
+        }
         soa.allocate(3 * soa_stride() * sizeof(float));
-        scratch.allocate(sort_scratch_bytes(static_cast<int>(n)));
         status.allocate(sizeof(unsigned));
         for (DeviceBuffer* b : {&xs0, &vin, &pn}) b->allocate(f4b);
         tf4.allocate(E * f4_per_step() * f4b);
