@@ -994,12 +994,16 @@ k_resolve(const float4* __restrict__ x, const float4* __restrict__ vin, float4* 
     v[i] = vv;
 }
 
-// scatterFloat4ByStableId (pbf_solver_kernels.cu:418-427).
+// scatterFloat4ByStableId (pbf_solver_kernels.cu:418-427).  After a run that failed
+// the ids may be those of an earlier, larger set of particles, or of none: such
+// a value is left out, out holds n.
 __global__ void __launch_bounds__(kBlock)
 k_scatter_by_id(const float4* __restrict__ vals, const uint32_t* __restrict__ id,
                 float4* __restrict__ out, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[id[i]] = vals[i];
+    if (i >= n) return;
+    const uint32_t o = id[i];
+    if (o < static_cast<uint32_t>(n)) out[o] = vals[i];
 }
 
 __global__ void __launch_bounds__(kBlock) k_iota(uint32_t* a, int n) {
