@@ -1011,19 +1011,25 @@ __global__ void __launch_bounds__(kBlock) k_iota(uint32_t* a, int n) {
     if (i < n) a[i] = static_cast<uint32_t>(i);
 }
 
-// |rho/rho0 - 1| per particle over the current lists.
+// |rho/rho0 - 1| per particle over the current lists.  A run that failed may leave
+// counts whose compact lists were never placed or written: entries past the lists'
+// capacity or naming no particle slot (of slots) are left out.
 __global__ void __launch_bounds__(kBlock)
 k_density(const float4* __restrict__ x, const uint32_t* __restrict__ nbr,
-          const int* __restrict__ cnt, StepConst c, int n, float* __restrict__ err) {
+          const int* __restrict__ cnt, StepConst c, int n, uint32_t slots,
+          float* __restrict__ err) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 pi = x[i];
     const int count = min(cnt[i], c.max_nb);
     float wsum = c.k.c_poly6;
-    const uint32_t* list = nbr + nb_first(c, i);
-    const size_t step = nb_step(c);
+    const size_t list = nb_first(c, i), step = nb_step(c);
     for (int k = 0; k < count; ++k) {
-        const float4 pj = __ldg(&x[__ldg(&list[static_cast<size_t>(k) * step])]);
+        const size_t at = list + static_cast<size_t>(k) * step;
+        if (c.nb_off != nullptr && at >= c.nb_cap) break;
+        const uint32_t j = __ldg(&nbr[at]);
+        if (j >= slots) continue;
+        const float4 pj = __ldg(&x[j]);
         wsum = fadd(wsum, poly6(c.k, dist2(fsub(pi.x, pj.x), fsub(pi.y, pj.y), fsub(pi.z, pj.z))));
     }
     const float mass = c.scenes ? scene_of(c, i).mass : c.mass;
@@ -1332,8 +1338,9 @@ void launch_iota(uint32_t* a, int n, cudaStream_t st) {
     k_iota<<<blocks_for(n), kBlock, 0, st>>>(a, n);
 }
 void launch_density(const float4* x, const uint32_t* nbr, const int* cnt, const StepConst& c,
-                    int n, float* err, cudaStream_t st) {
-    k_density<<<blocks_for(n), kBlock, 0, st>>>(x, nbr, cnt, c, n, err);
+                    int n, size_t slots, float* err, cudaStream_t st) {
+    k_density<<<blocks_for(n), kBlock, 0, st>>>(x, nbr, cnt, c, n, static_cast<uint32_t>(slots),
+                                                err);
 }
 void launch_grid_keys(const float4* pos, uint32_t* keys, int n, const GridConst& g,
                       cudaStream_t st) {

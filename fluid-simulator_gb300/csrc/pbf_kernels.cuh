@@ -218,7 +218,7 @@ void launch_scatter_by_id(const float4* vals, const uint32_t* id, float4* out, i
                           cudaStream_t st);
 void launch_iota(uint32_t* a, int n, cudaStream_t st);
 void launch_density(const float4* x, const uint32_t* nbr, const int* cnt, const StepConst& c,
-                    int n, float* err, cudaStream_t st);
+                    int n, size_t slots, float* err, cudaStream_t st);
 
 // --- stage kernels for the standalone entry points -------------------------
 void launch_grid_keys(const float4* pos, uint32_t* keys, int n, const GridConst& g,

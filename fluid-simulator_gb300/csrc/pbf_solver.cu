@@ -1353,7 +1353,7 @@ pbf_status pbf_density_error(pbf_solver* s, double* mean, double* mxe) {
         s->use_device();
         const StepConst c = s->make_const();
         launch_density(s->f4[s->ix].as<float4>(), s->nbr.as<uint32_t>(), s->cnt.as<int>(), c,
-                       static_cast<int>(s->n), s->lam.as<float>(), s->stream);
+                       static_cast<int>(s->n), s->cap, s->lam.as<float>(), s->stream);
         cuda_check(cudaGetLastError());
         std::vector<float> err(s->n);
         cuda_check(cudaMemcpyAsync(err.data(), s->lam.get(), s->n * sizeof(float),
