@@ -839,6 +839,15 @@ struct pbf_adjoint {
         if (!stream) cuda_check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
         if (!h_sums) cuda_check(cudaMallocHost(&h_sums, 2 * sizeof(double)));
         clear_graphs();
+        // An allocation that fails leaves buffers of both sizes: nothing to run on.
+        struct Undo {
+            pbf_adjoint* a;
+            ~Undo() {
+                if (!a) return;
+                a->n = 0;
+                a->drop_forward();
+            }
+        } undo{this};
         n = count;
         max_nb = maxnb;
         subs = p.substeps;
@@ -932,6 +941,7 @@ struct pbf_adjoint {
         cuda_check(cudaStreamSynchronize(stream));
         ckpt = DeviceBuffer();
         drop_forward();
+        undo.a = nullptr;
     }
 
     // CollisionSystem setters for the differentiated step (kind 0 spheres, 1

@@ -27,3 +27,20 @@ def test_again_on_other_grids(pbf, scenes):
             np.testing.assert_array_equal(g, w)
         fresh.close()
     a.close()
+
+
+def test_initialize_that_runs_out_of_memory(pbf, scenes):
+    """The adjoint is as if never initialised, until an initialise succeeds."""
+    scene = scenes.dam_break(9, 9, 9, (2.0, 1.0, 1.0), seed=1)
+    pos, vel, _, _, prm, _ = scene
+    a = pbf.PBFAdjoint()
+    want = _rollout(a, scene, (2.0, 1.0, 1.0))
+    with pytest.raises(pbf.SolverRuntimeError, match="out of memory"):
+        a.initialize(len(pos), (0.0, 0.0, 0.0), (2.0, 1.0, 1.0), prm, max_neighbors=1 << 28)
+    with pytest.raises(pbf.LogicError):
+        a.forward(pos, vel, 1)
+    with pytest.raises(pbf.LogicError):
+        a.backward(pos, vel)
+    for g, w in zip(_rollout(a, scene, (2.0, 1.0, 1.0)), want):
+        np.testing.assert_array_equal(g, w)
+    a.close()
