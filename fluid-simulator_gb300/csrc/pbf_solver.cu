@@ -48,26 +48,45 @@ using namespace pbf;
 
 namespace {
 
-// Bytes from p to the end of the device allocation that holds it; 0 if there is
-// none.
-size_t allocation_left(const void* p) {
-    using GetRange = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
-    static const GetRange get = [] {
+// What the driver knows about a caller's pointer, by one query (the runtime's
+// attributes have no range; the two calls take 0.3 us more an array).
+struct PointerInfo {
+    bool managed = false;
+    int memory = 0, device = -1;  // CUmemorytype, ordinal
+    size_t left = 0;              // bytes from p to the end of its allocation, 0: none
+};
+PointerInfo pointer_info(const void* p) {
+    using Query = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Query query = [] {
         void* f = nullptr;
         cudaDriverEntryPointQueryResult found{};
-        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000,
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000,
                                              cudaEnableDefault, &found) != cudaSuccess ||
             found != cudaDriverEntryPointSuccess) {
             cudaGetLastError();
             f = nullptr;
         }
-        return reinterpret_cast<GetRange>(f);
+        return reinterpret_cast<Query>(f);
     }();
     const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
+    CUmemorytype memory{};
+    int device = -1;
+    unsigned managed = 0;
     CUdeviceptr base = 0;
     size_t size = 0;
-    if (!get || get(&base, &size, at) != CUDA_SUCCESS || at < base || at - base >= size) return 0;
-    return size - (at - base);
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE,
+                                  CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                                  CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                  CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* out[] = {&memory, &device, &managed, &base, &size};
+    PointerInfo r;
+    if (!query || query(5, what, out, at) != CUDA_SUCCESS) return r;
+    r.memory = static_cast<int>(memory);
+    r.device = device;
+    r.managed = managed != 0;
+    if (at >= base && at - base < size) r.left = size - (at - base);
+    return r;
 }
 
 constexpr int kDefaultMaxNeighbors = 256;  // kMaxNeighbors, src/pbf/pbf_solver.cu:12
@@ -986,22 +1005,15 @@ struct pbf_solver {
     // cudaMemcpy and its own checks; an array that reaches past the end of device
     // memory is refused here with the status that the copy gives it.
     bool kernel_can_use(const void* p, size_t count) const {
-        cudaPointerAttributes a{};
         if (reinterpret_cast<uintptr_t>(p) % sizeof(float4) != 0) return false;
-        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        if (!((a.type == cudaMemoryTypeDevice && a.device == device) ||
-              a.type == cudaMemoryTypeManaged))
-            return false;
-        const size_t left = allocation_left(p);
-        if (left >= count * sizeof(float4)) return true;
-        if (left == 0) return false;  // not known: the copy decides
+        const PointerInfo q = pointer_info(p);
+        if (!q.managed && !(q.memory == CU_MEMORYTYPE_DEVICE && q.device == device)) return false;
+        if (q.left >= count * sizeof(float4)) return true;
+        if (q.left == 0) return false;  // not known: the copy decides
         // Past its allocation, but in the next ones all the way: mappings side by
         // side may hold one array, and the copy decides.
-        for (size_t at = left; at < count * sizeof(float4);) {
-            const size_t more = allocation_left(static_cast<const char*>(p) + at);
+        for (size_t at = q.left; at < count * sizeof(float4);) {
+            const size_t more = pointer_info(static_cast<const char*>(p) + at).left;
             if (more == 0) cuda_check(cudaErrorInvalidValue);
             at += more;
         }
