@@ -225,7 +225,7 @@ __device__ __forceinline__ void test_groups(Test test4, int j0, int left, uint32
 // (soa_stride_for), so a chunk may read past the last particle.  All lanes of
 // the warp take every row and chunk step together (active: the lane has a
 // particle), and hits is called by all of them.
-template <bool B, class Hits>
+template <bool B, bool WIDE, class Hits>
 __device__ __forceinline__ void for_each_chunk(const StepConst& c, int i, bool active, float4 pi,
                                                const float* __restrict__ sx,
                                                const float* __restrict__ sy,
@@ -258,12 +258,17 @@ __device__ __forceinline__ void for_each_chunk(const StepConst& c, int i, bool a
         acc = __funnelshift_l(__float_as_uint(b0), acc, 1);
         acc = __funnelshift_l(__float_as_uint(b1), acc, 1);
     };
-    // Steps of the warp: the radius, as far as the grid has rows (a stage call's
-    // radius may reach far past a thin grid); of the warp's scenes.
-    int Rz = min(rows.g.radius, rows.g.gz - 1), Ry = min(rows.g.radius, rows.g.gy - 1);
-    if constexpr (B) {
-        Rz = __reduce_max_sync(0xffffffffu, Rz);
-        Ry = __reduce_max_sync(0xffffffffu, Ry);
+    // Steps of the warp: the largest radius of its scenes.  WIDE (a stage call's
+    // radius of several cells, one grid): as far as the grid has rows, or a radius
+    // that reaches far past a thin grid would never end.  With the step's radius of
+    // one cell two bounds cost 0.2 to 0.4 % of a frame and save 1 % where the grid
+    // is one cell thick.
+    int Rz, Ry;
+    if constexpr (WIDE) {
+        Rz = min(rows.g.radius, rows.g.gz - 1);
+        Ry = min(rows.g.radius, rows.g.gy - 1);
+    } else {
+        Rz = Ry = __reduce_max_sync(0xffffffffu, rows.g.radius);
     }
     for (int dz = -Rz; dz <= Rz; ++dz)
         for (int dy = -Ry; dy <= Ry; ++dy) {
@@ -361,7 +366,7 @@ inline size_t queue_bytes(int threads) { return sizeof(uint2) * kQueue * threads
 // 65,536 particles, 76 -> 58 at 262,144, 280 -> 206 at 1,048,576 and 875 -> 688
 // for 256 batched scenes; the final walk with XSPH at 1,048,576 310 -> 248 (72
 // registers; 64 spill: +3 %).
-template <bool B, bool ALLOC, class T, class Load, class Use2, class Use1>
+template <bool B, bool ALLOC, bool WIDE, class T, class Load, class Use2, class Use1>
 __device__ __forceinline__ int walk_terms(const StepConst& c, int i, bool active, float4 pi,
                                           const float* __restrict__ sx,
                                           const float* __restrict__ sy,
@@ -412,7 +417,7 @@ __device__ __forceinline__ int walk_terms(const StepConst& c, int i, bool active
     };
 #pragma unroll 1
     for (;;) {
-        for_each_chunk<B>(c, i, active, pi, sx, sy, sz, first, [&](int j0, uint32_t bits) {
+        for_each_chunk<B, WIDE>(c, i, active, pi, sx, sy, sz, first, [&](int j0, uint32_t bits) {
             if (bits) {
                 if (!ALLOC || tail != end_of_queue) {
                     *tail = make_uint2(static_cast<uint32_t>(j0) + 31u, bits);
@@ -438,7 +443,7 @@ __device__ __forceinline__ int walk_terms(const StepConst& c, int i, bool active
     return count;
 }
 
-template <bool LAMBDA, bool B, bool ALLOC>
+template <bool LAMBDA, bool B, bool ALLOC, bool WIDE = false>
 __global__ void __launch_bounds__(kMaxTunedBlock)
 k_search(const float4* __restrict__ xs, const float* __restrict__ sx,
          const float* __restrict__ sy, const float* __restrict__ sz, const int* __restrict__ first,
@@ -452,7 +457,7 @@ k_search(const float4* __restrict__ xs, const float* __restrict__ sx,
     const float4 pi = xs[i];
     const f32x2 px = splat2(pi.x), py = splat2(pi.y), pz = splat2(pi.z);
     LambdaAcc acc{c.k.c_poly6, 0.0f, 0.0f, 0.0f, 0.0f};
-    const int count = walk_terms<B, ALLOC, float4>(
+    const int count = walk_terms<B, ALLOC, WIDE, float4>(
         c, i, active, pi, sx, sy, sz, first, nbr, c.max_nb,
         [&](uint32_t j) { return LAMBDA ? __ldg(&xs[j]) : float4{}; },
         [&](const float4& a, const float4& b) {
@@ -487,7 +492,7 @@ k_count(const float4* __restrict__ xs, const float* __restrict__ sx,
     const bool active = i < n;
     i = min(i, n - 1);
     int count = 0;
-    for_each_chunk<B>(c, i, active, xs[i], sx, sy, sz, first,
+    for_each_chunk<B, false>(c, i, active, xs[i], sx, sy, sz, first,
                       [&](int, uint32_t bits) { count += __popc(bits); });
     if (!active) return;
     cnt[i] = count;
@@ -854,7 +859,7 @@ k_search_xsph(const float4* __restrict__ xs, const float* __restrict__ sx,
     i = min(i, n - 1);
     const float4 pi = xs[i], vi = v[i];
     XsphAcc s{0.0f, 0.0f, 0.0f};
-    const int count = walk_terms<B, ALLOC, PosVel>(
+    const int count = walk_terms<B, ALLOC, false, PosVel>(
         c, i, active, pi, sx, sy, sz, first, nbr, c.max_nb,
         [&](uint32_t j) { return PosVel{__ldg(&xs[j]), __ldg(&v[j])}; },
         [&](const PosVel& a, const PosVel& b) { xsph_add2(c.k, s, pi, vi, a, b); },
@@ -1212,6 +1217,7 @@ void launch_search(const float4* xs, const float* sx, const float* sy, const flo
         launch_count_and_scan(xs, sx, sy, sz, first, c, n, cnt, status, st);
     }
     if (with_lambda) walk(b ? k_search<true, true, false> : k_search<true, false, false>);
+    else if (!b && c.g.radius > 1) walk(k_search<false, false, false, true>);
     else walk(b ? k_search<false, true, false> : k_search<false, false, false>);
 }
 
