@@ -515,9 +515,9 @@ def batched(pkg, scenes, steps: int, warmup: int, per_scene_steps: int):
             a.synchronize()
         return time.perf_counter() - t0
 
-    # Each baseline takes its better walk setting: the size rule (scenes below
-    # 32,768 particles split their walks over 8 or 4 lanes, best for one scene
-    # at a time) or 1 lane per particle (best when many solvers share the GPU).
+    # Each baseline takes its better walk setting: the size rule (scenes of up to
+    # 18,432 particles take 8 to 32 lanes a particle, best for one scene at a
+    # time) or 1 lane per particle (best when many solvers share the GPU).
     timed = {}
     for lanes in (0, 1):
         for a in solvers:

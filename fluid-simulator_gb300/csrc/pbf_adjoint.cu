@@ -681,11 +681,12 @@ inline unsigned grid_lanes(int n, int L) {
     return static_cast<unsigned>((static_cast<size_t>(n) * L + kB - 1) / kB);
 }
 // Lanes per particle of the gather passes: four below 2^17 particles, two
-// above.  The lanes set the order of the partial sums, so another number
-// rounds the gradients differently (3e-7 relative in the parameter
-// derivatives); backward of 4 steps (us) at 2 / 4 / 8 / 16 lanes: 528 / 373 /
-// 300 / 303 at 4,080 particles, 518 / 436 / 460 / 587 at 16,384, 850 / 961 /
-// 1,123 / 1,650 at 65,536, 2,563 / 2,794 / 3,624 / 5,833 at 262,144.
+// above.  The line is kept for the results, not for the time: the lanes set the
+// order of the partial sums, and another number rounds the gradients differently
+// (3e-7 relative in the parameter derivatives).  By time it would lie lower:
+// backward of 4 steps (us) at 2 / 4 / 8 / 16 lanes 528 / 373 / 300 / 303 at 4,080
+// particles, 518 / 436 / 460 / 587 at 16,384, 850 / 961 / 1,123 / 1,650 at 65,536,
+// 2,563 / 2,794 / 3,624 / 5,833 at 262,144.
 constexpr int kLanesBelow = 1 << 17;
 inline int lanes_for(int n) { return n < kLanesBelow ? kLanes : 2; }
 

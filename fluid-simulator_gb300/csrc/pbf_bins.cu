@@ -129,9 +129,11 @@ constexpr int kScanThreads = 512;
 // cells: 8.4 -> 5.4 us), kMany above.  The tiles' sums are counted with the keys
 // (put_key), a warp's particles of a tile at once, where the particles are in the
 // last rebuild's order and at most kTileCountMax: frame at 65,536 particles 244 ->
-// 238 us, pass at 262,144 (two substeps) 2,174 -> 2,150; at 8,388,608 the atomics
-// cost more than they save (13.6 -> 14.2 ms), and with particles in any order
-// neighbouring threads share no tile (200,003 positions 31 -> 70 us).  Else
+// 238 us, pass at 262,144 (two substeps) 2,174 -> 2,150.  At 8,388,608 the atomics
+// cost more than they save (13.6 -> 14.2 ms), at 1,048,576 still a little less
+// (four frames 7,589 -> 7,542 us); the line was drawn above the two sizes timed at
+// first.  With particles in any order neighbouring threads share no tile
+// (200,003 positions 31 -> 70 us).  Else
 // k_bin_sums reads the counts (5.0 us at 1,048,576 particles) or, up to
 // kDirectCells, every scan block those before its own tile (at 32,768 cells 5.4 us
 // against 3.8 + 5.9).

@@ -116,9 +116,6 @@ __device__ __forceinline__ void slab_dist2(float p, float lo, float cell, int k,
     above = d1 * d1;
 }
 
-// The neighbour walk of particle i (position pi): writes the list slot-major
-// at out[slot * stride] (at most cap entries) and returns the full count.
-// STORE = false counts the hits without writing the list.
 // The stencil rows of particle i, as the walks visit them: z0..z1 x y0..y1
 // (clamped to the grid), and range(z, y) gives row (z, y)'s candidate index
 // range [s, e): its cells x0..x1 are consecutive keys.  Keys fit in 32 bits

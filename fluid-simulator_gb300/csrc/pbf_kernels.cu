@@ -37,8 +37,9 @@ void launch_error_check(cudaError_t e) { cuda_check(e); }
 
 // Register cap of a neighbour-loop kernel bound by the latency of its
 // dependent gathers (list index, then the neighbour's data): fewer registers
-// a thread, more warps in flight (k_delta_apply: 58 -> 48 registers, no
-// spills, 6 % faster at 1M particles).
+// a thread, more warps in flight (k_delta_apply: 58 -> 48 registers, 6 % faster
+// at 1M particles; no spills with the exponents 1 to 4, 4 bytes batched, 16 to 20
+// with the exponent read at run time).
 #define PBF_GATHER_REGS(r) __maxnreg__(r)
 
 
@@ -364,8 +365,8 @@ inline size_t queue_bytes(int threads) { return sizeof(uint2) * kQueue * threads
 // any is full (lanes that empty theirs by themselves: walk 30 to 80 % longer in
 // dense scenes).  Walk and lambda, before and with all of this: 38 -> 28 us at
 // 65,536 particles, 76 -> 58 at 262,144, 280 -> 206 at 1,048,576 and 875 -> 688
-// for 256 batched scenes; the final walk with XSPH at 1,048,576 310 -> 248 (72
-// registers; 64 spill: +3 %).
+// for 256 batched scenes; the final walk with XSPH at 1,048,576 310 -> 248 (at 72
+// registers, with 4 to 12 bytes of spills; at 64 with more of them: +3 %).
 template <bool B, bool ALLOC, bool WIDE, class T, class Load, class Use2, class Use1>
 __device__ __forceinline__ int walk_terms(const StepConst& c, int i, bool active, float4 pi,
                                           const float* __restrict__ sx,
@@ -1158,7 +1159,9 @@ inline int group_lanes(const StepConst& c, int n) {
 // out the last wave once there are several blocks an SM: frame at 256 / 128 /
 // 64 threads 358 / 329 / 331 us at 131,072 particles, 608 / 593 / 598 at
 // 262,144, 1,837 / 1,806 / 1,829 at 1,048,576, 6.70 / 6.66 / 6.68 ms for 256
-// batched scenes; 242 / 242 / 241 at 65,536 and 202 / 210 / 215 at 32,768.
+// batched scenes.  Near the line 256 and 128 threads win in turn, as their blocks
+// fill whole waves: 187 / 195 at 24,576, 198 / 202 at 32,768, 204 / 207 at 40,960,
+// 214 / 212 at 45,056, 223 / 217 at 57,344, 226 / 231 at 65,536, 260 / 246 at 81,920.
 constexpr size_t kBlock128From = 57344;
 int default_block(size_t n, int lanes) {
     if (lanes > 1) return kGroupBlock;

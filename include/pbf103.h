@@ -101,7 +101,9 @@ pbf_status pbf_initialize_compact(pbf_solver* s, size_t max_particles, pbf_float
  * finiteness checked, stable ids reset to the given order. */
 pbf_status pbf_set_particles(pbf_solver* s, const pbf_float4* positions,
                              const pbf_float4* velocities, size_t count);
-/* Same from device pointers (float4 arrays already resident in HBM). */
+/* Same from device pointers (float4 arrays already resident in HBM).  An array that
+ * runs past the end of device memory is refused with PBF_ERR_RUNTIME, with the
+ * particles as they were; so is a short destination of the device copies below. */
 pbf_status pbf_set_particles_device(pbf_solver* s, const pbf_float4* d_positions,
                                     const pbf_float4* d_velocities, size_t count);
 
